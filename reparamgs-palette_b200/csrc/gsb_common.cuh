@@ -36,9 +36,9 @@ constexpr float SH_C3_3 = 0.3731763325901154f;
 constexpr float SH_C3_5 = 1.445305721320277f;
 
 // Margin (in Mahalanobis units) added to the exact skip threshold
-// 2 ln(alpha / 0.002): a pixel farther than the cut is guaranteed to give
-// alpha' < 0.002 in the reference's own FP32 evaluation, so skipping it never
-// changes a result; pixels inside it are evaluated exactly as the reference.
+// 2 ln(alpha / 0.002) for the culling cut: a pixel farther than the cut is
+// guaranteed to give alpha' < 0.002 in the reference's own FP32 evaluation, so
+// culling it never changes a result.
 constexpr float kCutMargin = 1e-3f;
 
 inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
@@ -60,15 +60,18 @@ __device__ __forceinline__ float ld(const __nv_bfloat16* p, int64_t i) {
 // The intrinsics are never re-contracted, so the forward and the adjoint
 // (separate kernels) take the same skip (alpha' < 0.002) and stop
 // (T < 1e-4) decisions as the reference and as each other.
-__device__ __forceinline__ float maha_sq(float qa, float qb, float qc, float dx, float dy) {
-  const float cross = __fmul_rn(__fmul_rn(2.f, qb), dx);
-  return __fmaf_rn(cross, dy, __fmaf_rn(__fmul_rn(qa, dx), dx, __fmul_rn(__fmul_rn(qc, dy), dy)));
+// The form is evaluated as p = -m / 2 from the record's scaled conic (a = -qa
+// / 2, b = -qb, c = -qc / 2): powers of two scale through every rounding, so p
+// is exactly -1/2 of the reference's m.
+__device__ __forceinline__ float half_form(float a, float b, float c, float dx, float dy) {
+  return __fmaf_rn(__fmul_rn(b, dx), dy,
+                   __fmaf_rn(__fmul_rn(a, dx), dx, __fmul_rn(__fmul_rn(c, dy), dy)));
 }
 
 // Packed per-Gaussian record read by the compositing kernels (layout in
-// gsb_record.cuh): float4 v0 = centre and conic a, b; v1 = conic c, skip
-// cut, opacity, channel 0; v2 = support half-extents and the conic
-// diagonal's reciprocals; v3.. = channels 1..K-1, zero padded.
+// gsb_record.cuh): float4 v0 = centre and scaled conic a, b; v1 = conic c, skip
+// threshold, opacity, channel 0; v2 = support half-extents and cut; v3.. =
+// channels 1..K-1, zero padded.
 template <int K>
 struct RecordLayout {
   static constexpr int kFloats = ((11 + K) + 3) / 4 * 4;

@@ -105,7 +105,9 @@ int launch_sort_capacity(const SortPlan& p, int64_t n, int H, int W, const Splat
                          void* ws, int32_t* gsid_out, int32_t* ranges_out, uint32_t* status,
                          cudaStream_t st);
 
-// raster.cu
+// raster.cu, raster_backward.cu
+// Launch order of the compositing tiles, longest list first.
+int launch_tile_order(const int2* ranges, int tiles, int32_t* order, cudaStream_t st);
 int launch_draw(int64_t n, int H, int W, int channels, const int32_t* ranges, const int32_t* gsid,
                 const SplatState& s, float tau_init, float* out, int32_t* contrib,
                 float* final_tau, cudaStream_t st);
