@@ -4,14 +4,18 @@
 // One 128-thread block per 16x16 tile; each of the 4 warps owns an 8x8 block
 // and each lane two pixels of one column, four rows apart, so the
 // per-Gaussian loop control and the warp reduction of the gradient terms are
-// shared by 64 pixels.  Batches are staged and culled as in the forward: each
-// record's mask of the quarters its cut ellipse can reach is found once, by
-// the thread that stages it.  The warps walk their records from the last
-// contributor to the front, two at a time: both records' opacity terms are
-// evaluated before the two transmittance recoveries so that their exp()
-// chains overlap, and the two records' gradient vectors are summed in one
-// warp reduction.  Masks at staging and the exact skip threshold: 0.364 ->
-// 0.329 ms at 1M Gaussians, 1080p (full adjoint, 500k: 0.609 -> 0.581 ms).
+// shared by 64 pixels (few tiles: 8 warps, one pixel per lane, kOnePixelTiles).
+// Batches are staged and culled as in the forward: each record's mask of the
+// blocks its cut ellipse can reach is found once, by the thread that stages it.
+// The warps walk their records from the last contributor to the front, two at a
+// time: both records' opacity terms are evaluated before the two transmittance
+// recoveries so that their exp() chains overlap, and the two records' gradient
+// vectors are summed in one warp reduction.  What bounds it: instruction issue
+// (87 % with weights only, 79 % in the full adjoint).  At 1M Gaussians, 1080p:
+// 0.364 -> 0.329 ms with the masks at staging and the exact skip threshold, ->
+// 0.315 ms with T recovered by one approximate reciprocal and the exact-width
+// reduction; full adjoint (500k, K = 5): 0.609 -> 0.581 -> 0.455 ms, also with
+// the scalar recursion and the moments (adjoint_pixel).
 #include "gsb_geometry.cuh"
 #include "gsb_internal.h"
 #include "gsb_tiles.cuh"
@@ -19,25 +23,15 @@
 namespace gsb {
 
 constexpr int kBatch = 256;
-constexpr int kAdjThreads = 128;  // two pixels per thread, 8x8 pixels per warp
 
-struct PixelPair {
-  int tx, ty;    // tile origin; the warp blocks are its 8x8 quarters
-  int px;        // column
-  int py0, py1;  // rows (py1 = py0 + 4)
+// Pixels of a lane: NP of one column, four rows apart.  NP = 2: 4 warps per
+// tile, 8x8 pixels each; NP = 1: 8 warps, 8x4 pixels each.
+template <int NP>
+struct AdjLayout {
+  static constexpr int kThreads = kTilePixels / NP;
+  static constexpr int kRows = 4 * NP;             // rows of a warp's block
+  static constexpr int kBands = kTile / kRows;     // of two blocks of 8 columns each
 };
-
-__device__ __forceinline__ PixelPair pixels_of(int tile, int gx) {
-  const int tx = tile % gx, ty = tile / gx;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  PixelPair p;
-  p.tx = tx * kTile;
-  p.ty = ty * kTile;
-  p.px = p.tx + (w & 1) * 8 + (lane & 7);
-  p.py0 = p.ty + (w >> 1) * 8 + (lane >> 3);
-  p.py1 = p.py0 + 4;
-  return p;
-}
 
 template <int K>
 __device__ __forceinline__ void load_feats(const float4* srec, int j, float v2w, float* f) {
@@ -49,83 +43,93 @@ __device__ __forceinline__ void load_feats(const float4* srec, int j, float v2w,
   }
 }
 
-// Sum of NV per-lane values over groups of 2*OFF0 lanes (the whole warp for
-// OFF0 = 16, each half-warp for OFF0 = 8) with NV-1 + log2(2*OFF0/NV)
-// shuffles: each exchange step halves the values a lane carries (lanes with
-// the step's bit set keep the upper half), so the totals end up spread over
-// the group's lanes.  Returns this lane's total; *idx is the value index it
-// holds and *owner is set on exactly one lane per index and group.
-template <int NV, int OFF0 = 16>
-__device__ __forceinline__ float warp_transpose_sum(float (&x)[NV], int lane, int* idx,
-                                                    bool* owner) {
-  static_assert(NV >= 1 && NV <= 2 * OFF0 && (NV & (NV - 1)) == 0,
-                "NV must be a power of two no larger than the group");
-  int id = 0;
-  int off = OFF0;
+// Sum of N per-lane values over groups of 2 * OFF lanes, spread over the
+// group's lanes: each exchange step halves the values a lane carries (lanes
+// with the step's bit set keep the upper half), so 11 values take 6 + 3 + 2 + 1
+// shuffles instead of the 8 + 4 + 2 + 1 of 16 padded ones.  Returns this lane's
+// total; *idx is the value it holds, *owner is set on one lane per value and
+// group.
+template <int N, int OFF>
+__device__ __forceinline__ float warp_spread_sum(float* x, int lane, int* idx, bool* owner) {
+  constexpr int kHalf = (N + 1) / 2;
+  const bool hi = (lane & OFF) != 0;
+  if constexpr (N > 1) {
 #pragma unroll
-  for (int w = NV / 2; w >= 1; w >>= 1, off >>= 1) {
-    const bool hi = (lane & off) != 0;
-#pragma unroll
-    for (int i = 0; i < w; ++i) {
-      const float send = hi ? x[i] : x[i + w];
-      const float keep = hi ? x[i + w] : x[i];
-      x[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    for (int i = 0; i < kHalf; ++i) {
+      const float other = kHalf + i < N ? x[kHalf + i < N ? kHalf + i : 0] : 0.f;
+      x[i] = (hi ? other : x[i]) + __shfl_xor_sync(0xffffffffu, hi ? x[i] : other, OFF);
     }
-    id += hi ? w : 0;
-  }
-  float v = x[0];
+    int at = 0;
+    bool own = true;
+    float v = x[0];
+    if constexpr (OFF > 1)
+      v = warp_spread_sum<kHalf, OFF / 2>(x, lane, &at, &own);
+    else
+      static_assert(N <= 2, "more values than lanes");
+    *idx = at + (hi ? kHalf : 0);
+    *owner = own && at < (hi ? N - kHalf : kHalf);
+    return v;
+  } else {
+    float v = x[0];
 #pragma unroll
-  for (int o = off; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  *idx = id;
-  *owner = off == 0 || (lane & (2 * off - 1)) == 0;  // NV == group size: every lane
-  return v;
+    for (int o = OFF; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    *idx = 0;
+    *owner = (lane & (2 * OFF - 1)) == 0;
+    return v;
+  }
 }
-
-template <int NV>
-struct Pow2 {
-  static constexpr int value = NV <= 1 ? 1 : NV <= 2 ? 2 : NV <= 4 ? 4 : NV <= 8 ? 8 : NV <= 16 ? 16 : 32;
-};
 
 // Per-pixel back-to-front state of the adjoint.
 template <int K>
 struct BwdPixel {
-  float dl[K], G[K];
-  float T, Tf, dTf;
+  float dl[K];
+  float T, R;  // R: dl . (what is blended behind), the full adjoint's
   int cont;
 };
 
 // One contributor of one pixel in the adjoint: recovers T, accumulates the
-// pixel's gradient terms into x (x[0..K) features, then alpha, u, conic).
-template <int K, bool GEOM, bool DTAU>
-__device__ __forceinline__ bool adjoint_pixel(BwdPixel<K>& p, int idx, float m, float4 v0,
-                                              float4 v1, float dx, float dy, const float4* srec,
-                                              int jj, float* x) {
+// pixel's gradient terms into x: x[0..K) features, then (GEOM) alpha and the
+// moments h d, h d d^T of h = dL/dalpha' alpha' (finish_geom).  With s = dl . f,
+// dL/dalpha' = T (s - R), where R is the blended s of everything behind the
+// record: one scalar recursion instead of one per channel (0.565 -> 0.481 ms
+// at 500k Gaussians, 1080p, K = 5, with the moments).
+template <int K, bool GEOM>
+__device__ __forceinline__ bool adjoint_pixel(BwdPixel<K>& p, int idx, float m, float4 v1,
+                                              float dx, float dy, const float* f, float* x) {
   if (!(idx < p.cont) || !(m >= v1.y)) return false;
   const float g = expf(m);
   const float ap = fminf(kAlphaMax, v1.z * g);
-  const float one_m = 1.f - ap;
-  p.T = __fdividef(p.T, one_m);
+  p.T *= rcp_approx(1.f - ap);
   const float wgt = ap * p.T;
 #pragma unroll
   for (int k = 0; k < K; ++k) x[k] += p.dl[k] * wgt;
-  if (GEOM) {
-    float f[K];
-    load_feats<K>(srec, jj, v1.w, f);
-    float dap = 0.f;
+  if constexpr (GEOM) {
+    float s = p.dl[0] * f[0];
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      dap += p.dl[k] * (p.T * (f[k] - p.G[k]));
-      p.G[k] = ap * f[k] + one_m * p.G[k];
-    }
-    if (DTAU) dap += p.dTf * __fdividef(-p.Tf, one_m);
-    x[K] += dap * g;                                    // alpha
-    x[K + 1] += dap * ((2.f * v0.z * dx + v0.w * dy) * ap);  // u.x
-    x[K + 2] += dap * ((v0.w * dx + 2.f * v1.x * dy) * ap);  // u.y
-    x[K + 3] += dap * (-0.5f * ap * (dx * dx));         // conic a
-    x[K + 4] += dap * (-1.0f * ap * (dx * dy));         // conic b
-    x[K + 5] += dap * (-0.5f * ap * (dy * dy));         // conic c
+    for (int k = 1; k < K; ++k) s += p.dl[k] * f[k];
+    const float t = s - p.R;
+    const float dap = p.T * t;
+    p.R = fmaf(ap, t, p.R);
+    const float h = dap * ap, tx = h * dx, ty = h * dy;
+    x[K] += dap * g;
+    x[K + 1] += tx;
+    x[K + 2] += ty;
+    x[K + 3] += tx * dx;
+    x[K + 4] += tx * dy;
+    x[K + 5] += ty * dy;
   }
   return true;
+}
+
+// The lane's moments to its centre (K + 1, K + 2) and conic gradients.
+template <int K>
+__device__ __forceinline__ void finish_geom(float4 v0, float4 v1, float* x) {
+  const float Sx = x[K + 1], Sy = x[K + 2];
+  x[K + 1] = 2.f * v0.z * Sx + v0.w * Sy;
+  x[K + 2] = v0.w * Sx + 2.f * v1.x * Sy;
+  x[K + 3] *= -0.5f;
+  x[K + 4] = -x[K + 4];
+  x[K + 5] *= -0.5f;
 }
 
 // Weights-only adjoint of two contributors at once: slot ja lies behind slot
@@ -134,26 +138,26 @@ __device__ __forceinline__ bool adjoint_pixel(BwdPixel<K>& p, int idx, float m, 
 // exp() chains overlap; the skip tests and the T recovery are exactly those
 // of adjoint_pixel.  The two gradient vectors are summed together: one
 // exchange at offset 16 leaves ja's partial sums on lanes 0-15 and jb's on
-// lanes 16-31, then each half-warp transposes its K values (5 + 8 shuffles
-// for K = 5, against 2 x 9 for two single reductions).  When at most
-// kDirectLanes lanes hit each record, those lanes add their own sums
+// lanes 16-31, then each half-warp spreads its K values (5 + 7 shuffles for
+// K = 5).  When at most kDirectLanes lanes hit each record, those lanes add
+// their own sums
 // directly (at most 2 x kDirectLanes x K atomics instead of about 60
 // reduction instructions; 47 % of the records a warp visits have so few hits
 // at 1M Gaussians, 1080p).  Measured, near / far view: 4 lanes 0.367 / 0.282
 // ms, 8 lanes 0.362 / 0.278, 12 lanes 0.360 / 0.275, 16 lanes 0.361 / 0.278.
 constexpr int kDirectLanes = 12;
-template <int K>
-__device__ __forceinline__ void adjoint_weights_pair(BwdPixel<K> (&p)[2], int base, int ja, int jb,
-                                                     const float4* srec, const int32_t* sgid,
-                                                     float fx, float fy0, float fy1, int lane,
+template <int K, int NP>
+__device__ __forceinline__ void adjoint_weights_pair(BwdPixel<K> (&p)[NP], int base, int ja,
+                                                     int jb, const float4* srec,
+                                                     const int32_t* sgid, float fx,
+                                                     const float (&fy)[NP], int lane,
                                                      float* __restrict__ dfeat) {
   const float4 a0 = srec[ja], a1 = srec[kBatch + ja];
   const float4 b0 = srec[jb], b1 = srec[kBatch + jb];
-  const float fy[2] = {fy0, fy1};
-  float apa[2], apb[2];
-  bool ua[2], ub[2];
+  float apa[NP], apb[NP];
+  bool ua[NP], ub[NP];
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
+  for (int q = 0; q < NP; ++q) {
     const float dxa = a0.x - fx, dya = a0.y - fy[q];
     const float ma = fminf(0.f, half_form(a0.z, a0.w, a1.x, dxa, dya));
     apa[q] = fminf(kAlphaMax, a1.z * expf(ma));
@@ -167,24 +171,24 @@ __device__ __forceinline__ void adjoint_weights_pair(BwdPixel<K> (&p)[2], int ba
 #pragma unroll
   for (int k = 0; k < K; ++k) xa[k] = xb[k] = 0.f;
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
+  for (int q = 0; q < NP; ++q) {
     if (ua[q]) {
-      p[q].T = __fdividef(p[q].T, 1.f - apa[q]);
+      p[q].T *= rcp_approx(1.f - apa[q]);
       const float wgt = apa[q] * p[q].T;
 #pragma unroll
       for (int k = 0; k < K; ++k) xa[k] += p[q].dl[k] * wgt;
     }
   }
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
+  for (int q = 0; q < NP; ++q) {
     if (ub[q]) {
-      p[q].T = __fdividef(p[q].T, 1.f - apb[q]);
+      p[q].T *= rcp_approx(1.f - apb[q]);
       const float wgt = apb[q] * p[q].T;
 #pragma unroll
       for (int k = 0; k < K; ++k) xb[k] += p[q].dl[k] * wgt;
     }
   }
-  const bool ha = ua[0] || ua[1], hb = ub[0] || ub[1];
+  const bool ha = ua[0] || ua[NP - 1], hb = ub[0] || ub[NP - 1];
   const unsigned ca = __ballot_sync(0xffffffffu, ha), cb = __ballot_sync(0xffffffffu, hb);
   if (!(ca | cb)) return;
   if (__popc(ca) <= kDirectLanes && __popc(cb) <= kDirectLanes) {
@@ -200,23 +204,18 @@ __device__ __forceinline__ void adjoint_weights_pair(BwdPixel<K> (&p)[2], int ba
     }
     return;
   }
-  constexpr int NV = Pow2<K>::value;
   const bool hi = (lane & 16) != 0;
-  float y[NV];
+  float y[K];
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    if (k < K) {
-      const float send = hi ? xa[k] : xb[k];
-      const float keep = hi ? xb[k] : xa[k];
-      y[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-    } else {
-      y[k] = 0.f;
-    }
+  for (int k = 0; k < K; ++k) {
+    const float send = hi ? xa[k] : xb[k];
+    const float keep = hi ? xb[k] : xa[k];
+    y[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
   }
   int vidx;
   bool owner;
-  const float tot = warp_transpose_sum<NV, 8>(y, lane, &vidx, &owner);
-  if (owner && vidx < K && (hi ? cb : ca) != 0u) {
+  const float tot = warp_spread_sum<K, 8>(y, lane, &vidx, &owner);
+  if (owner && (hi ? cb : ca) != 0u) {
     const int64_t g = sgid[hi ? jb : ja];
     atomicAdd(dfeat + g * K + vidx, tot);
   }
@@ -237,38 +236,46 @@ __device__ __forceinline__ float* grad_slot(int v, int64_t g, float* dfeat, floa
 // the per-pixel terms are adjoint_pixel's, in the same order (ja then jb for
 // each pixel).  The two gradient vectors (K + 6 values each) are summed
 // together: one exchange at lane offset 16 leaves ja's partial sums on lanes
-// 0-15 and jb's on lanes 16-31, then each half-warp transposes its values
-// (K + 6 + 15 shuffles for the pair instead of 2 x 16 for K = 3..8).  When
+// 0-15 and jb's on lanes 16-31, then each half-warp spreads its values (11 + 12
+// shuffles for K = 5).  When
 // at most kDirectLanesGeom lanes hit each record, those lanes add their own
 // K + 6 sums directly: at 1M / 1080p 0.776 -> 0.755 ms near, 0.462 -> 0.439
 // ms far, against direct atomics for single hits only.
 constexpr int kDirectLanesGeom = 8;
-template <int K, bool DTAU>
-__device__ __forceinline__ void adjoint_geom_pair(BwdPixel<K> (&p)[2], int base, int ja, int jb,
+template <int K, int NP>
+__device__ __forceinline__ void adjoint_geom_pair(BwdPixel<K> (&p)[NP], int base, int ja, int jb,
                                                   const float4* srec, const int32_t* sgid,
-                                                  float fx, float fy0, float fy1, int lane,
+                                                  float fx, const float (&fy)[NP], int lane,
                                                   float* __restrict__ dfeat,
                                                   float* __restrict__ dalpha,
                                                   float* __restrict__ du,
                                                   float* __restrict__ dconic) {
   constexpr int NREAL = K + 6;
-  constexpr int NV = Pow2<NREAL>::value;
-  static_assert(NV <= 16, "half-warp transposition holds at most 16 values");
   const float4 a0 = srec[ja], a1 = srec[kBatch + ja];
   const float4 b0 = srec[jb], b1 = srec[kBatch + jb];
-  float xa[NV], xb[NV];
+  float xa[NREAL], xb[NREAL];
 #pragma unroll
-  for (int v = 0; v < NV; ++v) xa[v] = xb[v] = 0.f;
-  const float dxa = a0.x - fx, dya0 = a0.y - fy0, dya1 = a0.y - fy1;
-  const float dxb = b0.x - fx, dyb0 = b0.y - fy0, dyb1 = b0.y - fy1;
-  const float ma0 = fminf(0.f, half_form(a0.z, a0.w, a1.x, dxa, dya0));
-  const float ma1 = fminf(0.f, half_form(a0.z, a0.w, a1.x, dxa, dya1));
-  const float mb0 = fminf(0.f, half_form(b0.z, b0.w, b1.x, dxb, dyb0));
-  const float mb1 = fminf(0.f, half_form(b0.z, b0.w, b1.x, dxb, dyb1));
-  bool ha = adjoint_pixel<K, true, DTAU>(p[0], base + ja, ma0, a0, a1, dxa, dya0, srec, ja, xa);
-  bool hb = adjoint_pixel<K, true, DTAU>(p[0], base + jb, mb0, b0, b1, dxb, dyb0, srec, jb, xb);
-  ha |= adjoint_pixel<K, true, DTAU>(p[1], base + ja, ma1, a0, a1, dxa, dya1, srec, ja, xa);
-  hb |= adjoint_pixel<K, true, DTAU>(p[1], base + jb, mb1, b0, b1, dxb, dyb1, srec, jb, xb);
+  for (int v = 0; v < NREAL; ++v) xa[v] = xb[v] = 0.f;
+  const float dxa = a0.x - fx, dxb = b0.x - fx;
+  float dya[NP], dyb[NP], ma[NP], mb[NP];
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    dya[q] = a0.y - fy[q];
+    dyb[q] = b0.y - fy[q];
+    ma[q] = fminf(0.f, half_form(a0.z, a0.w, a1.x, dxa, dya[q]));
+    mb[q] = fminf(0.f, half_form(b0.z, b0.w, b1.x, dxb, dyb[q]));
+  }
+  float fa[K], fb[K];
+  load_feats<K>(srec, ja, a1.w, fa);
+  load_feats<K>(srec, jb, b1.w, fb);
+  bool ha = false, hb = false;
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    ha |= adjoint_pixel<K, true>(p[q], base + ja, ma[q], a1, dxa, dya[q], fa, xa);
+    hb |= adjoint_pixel<K, true>(p[q], base + jb, mb[q], b1, dxb, dyb[q], fb, xb);
+  }
+  finish_geom<K>(a0, a1, xa);
+  finish_geom<K>(b0, b1, xb);
   const unsigned ca = __ballot_sync(0xffffffffu, ha), cb = __ballot_sync(0xffffffffu, hb);
   if (!(ca | cb)) return;
   if (__popc(ca) <= kDirectLanesGeom && __popc(cb) <= kDirectLanesGeom) {
@@ -285,21 +292,17 @@ __device__ __forceinline__ void adjoint_geom_pair(BwdPixel<K> (&p)[2], int base,
     return;
   }
   const bool hi = (lane & 16) != 0;
-  float y[NV];
+  float y[NREAL];
 #pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    if (v < NREAL) {
-      const float send = hi ? xa[v] : xb[v];
-      const float keep = hi ? xb[v] : xa[v];
-      y[v] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-    } else {
-      y[v] = 0.f;
-    }
+  for (int v = 0; v < NREAL; ++v) {
+    const float send = hi ? xa[v] : xb[v];
+    const float keep = hi ? xb[v] : xa[v];
+    y[v] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
   }
   int vidx;
   bool owner;
-  const float tot = warp_transpose_sum<NV, 8>(y, lane, &vidx, &owner);
-  if (owner && vidx < NREAL && (hi ? cb : ca) != 0u) {
+  const float tot = warp_spread_sum<NREAL, 8>(y, lane, &vidx, &owner);
+  if (owner && (hi ? cb : ca) != 0u) {
     const int64_t g = sgid[hi ? jb : ja];
     atomicAdd(grad_slot<K>(vidx, g, dfeat, dalpha, du, dconic), tot);
   }
@@ -313,14 +316,16 @@ __device__ __forceinline__ void adjoint_geom_pair(BwdPixel<K> (&p)[2], int base,
 // Gaussian each lane first adds its two pixels' terms, then the warp's 64
 // pixels are summed with one transposed reduction and added with one atomic
 // per value.  GEOM adds the opacity / centre / conic adjoint (draw_color_B's
-// terms, for any channel count); DTAU adds dL/dT_final
-// (vanilla_3dgs/gsplatcu/kernel.cu:912-919).  As in the reference, the 0.99
-// clamp and max(0, .) are not differentiated.  Weights-only, 8 blocks per SM
-// (64 registers, a 12-byte spill): 0.377 -> 0.365 ms at 1M / 1080p against 7
-// blocks (72 registers); the full adjoint 6 blocks per SM (80 registers):
-// 0.755 -> 0.722 ms near, 1.146 -> 1.112 ms close, 0.437 -> 0.450 ms far.
-template <int K, bool GEOM, bool DTAU>
-__global__ void __launch_bounds__(kAdjThreads, GEOM ? 6 : 8)
+// terms, for any channel count); dL/dT_final (vanilla_3dgs/gsplatcu/kernel.cu:
+// 912-919) enters as the value of R behind the last contributor, since
+// d T_final / d alpha' = -T_final / (1 - alpha').  As in the reference, the 0.99
+// clamp and max(0, .) are not differentiated.  Weights-only 8 blocks of 128
+// threads per SM (61 registers); full adjoint 7 for K = 4 and 5 (0.476 ->
+// 0.462 ms at 500k, K = 5, against 6), 6 otherwise (K = 3: 0.364 against 0.371
+// ms at 7; above 5 channels 7 would spill 90 bytes).
+template <int K, bool GEOM, int NP>
+__global__ void __launch_bounds__(AdjLayout<NP>::kThreads,
+                                  (GEOM ? (K == 4 || K == 5 ? 7 : 6) : 8) * NP / 2)
     k_draw_backward(int H, int W, int gx, const int2* __restrict__ ranges,
                     const int32_t* __restrict__ gsid, const float4* __restrict__ records,
                     const int32_t* __restrict__ order,
@@ -329,37 +334,38 @@ __global__ void __launch_bounds__(kAdjThreads, GEOM ? 6 : 8)
                     float* __restrict__ dfeat, float* __restrict__ dalpha,
                     float* __restrict__ du, float* __restrict__ dconic) {
   pdl_wait();
+  using L = AdjLayout<NP>;
   constexpr int V = RecordLayout<K>::kVec4;
   constexpr int NREAL = GEOM ? K + 6 : K;
-  constexpr int NV = Pow2<NREAL>::value;
   constexpr int kKeep = GEOM ? V - 1 : 2;  // float4s kept (v0, v1 and, with GEOM, the further channels)
   __shared__ float4 srec[kKeep * kBatch];
   __shared__ int32_t sgid[kBatch];
   __shared__ uint8_t smask[kBatch];
   __shared__ unsigned s_maxc;
   const int tile = order[blockIdx.x];
-  const PixelPair pp = pixels_of(tile, gx);
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int X0 = (tile % gx) * kTile, Y0 = (tile / gx) * kTile;
+  const int px = X0 + (w & 1) * 8 + (lane & 7);
+  const int py = Y0 + (w >> 1) * L::kRows + (lane >> 3);
   const int2 rg = ranges[tile];
   if (rg.y - rg.x == 0) return;  // uniform per block
   const int64_t hw = (int64_t)H * W;
-  BwdPixel<K> p[2];
-  const int rows[2] = {pp.py0, pp.py1};
+  BwdPixel<K> p[NP];
+  float fy[NP];
+  int wmax = 0;
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const bool in = pp.px < W && rows[q] < H;
-    const int64_t pix = (int64_t)rows[q] * W + pp.px;
+  for (int q = 0; q < NP; ++q) {
+    const bool in = px < W && py + 4 * q < H;
+    const int64_t pix = (int64_t)(py + 4 * q) * W + px;
+    fy[q] = (float)(py + 4 * q);
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      p[q].dl[k] = in ? dout[k * hw + pix] : 0.f;
-      p[q].G[k] = 0.f;
-    }
-    p[q].Tf = in ? final_tau[pix] : 0.f;
-    p[q].T = p[q].Tf;
-    p[q].dTf = (DTAU && in) ? dtau[pix] : 0.f;
+    for (int k = 0; k < K; ++k) p[q].dl[k] = in ? dout[k * hw + pix] : 0.f;
+    p[q].T = in ? final_tau[pix] : 0.f;
+    p[q].R = (GEOM && dtau && in) ? dtau[pix] : 0.f;
     p[q].cont = in ? contrib[pix] : 0;
+    wmax = max(wmax, p[q].cont);
   }
-  const int wmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(p[0].cont, p[1].cont));
+  wmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)wmax);
   if (threadIdx.x == 0) s_maxc = 0u;
   __syncthreads();
   if (lane == 0) atomicMax(&s_maxc, (unsigned)wmax);
@@ -367,12 +373,12 @@ __global__ void __launch_bounds__(kAdjThreads, GEOM ? 6 : 8)
   // contributor indices never exceed the tile's list (clamped for safety
   // against mismatched inputs)
   const int maxc = min((int)s_maxc, rg.y - rg.x);
-  const float fx = (float)pp.px, fy0 = (float)pp.py0, fy1 = (float)pp.py1;
+  const float fx = (float)px;
   for (int top = maxc; top > 0; top -= kBatch) {
     const int base = max(0, top - kBatch);
     const int cnt = top - base;
     __syncthreads();
-    for (int t = threadIdx.x; t < cnt; t += kAdjThreads) {
+    for (int t = threadIdx.x; t < cnt; t += L::kThreads) {
       const int g = gsid[rg.x + base + t];
       const float4* src = records + (int64_t)g * V;
       const float4 v0 = __ldg(src), v1 = __ldg(src + 1), v2 = __ldg(src + 2);
@@ -382,14 +388,14 @@ __global__ void __launch_bounds__(kAdjThreads, GEOM ? 6 : 8)
       for (int v = 3; v < V; ++v)
         if (GEOM) srec[(v - 1) * kBatch + t] = __ldg(src + v);
       sgid[t] = g;
-      smask[t] = (uint8_t)region_mask<2, 2, 8, 8>(v0, v1, v2, pp.tx, pp.ty);
+      smask[t] = (uint8_t)region_mask<2, L::kBands, 8, L::kRows>(v0, v1, v2, X0, Y0);
     }
     __syncthreads();
     const int hi = min(cnt, wmax - base);
     for (int s_hi = hi; s_hi > 0; s_hi -= 32) {
       const int s_lo = max(0, s_hi - 32);
       const int j = s_lo + lane;
-      unsigned mask = __ballot_sync(0xffffffffu, j < s_hi && ((smask[j] >> (threadIdx.x >> 5)) & 1));
+      unsigned mask = __ballot_sync(0xffffffffu, j < s_hi && ((smask[j] >> w) & 1));
       while (mask) {
         const int msb = 31 - __clz(mask);
         mask &= ~(1u << msb);
@@ -397,74 +403,69 @@ __global__ void __launch_bounds__(kAdjThreads, GEOM ? 6 : 8)
           const int msb2 = 31 - __clz(mask);
           mask &= ~(1u << msb2);
           if constexpr (GEOM)
-            adjoint_geom_pair<K, DTAU>(p, base, s_lo + msb, s_lo + msb2, srec, sgid, fx, fy0, fy1,
-                                       lane, dfeat, dalpha, du, dconic);
+            adjoint_geom_pair<K, NP>(p, base, s_lo + msb, s_lo + msb2, srec, sgid, fx, fy, lane,
+                                       dfeat, dalpha, du, dconic);
           else
-            adjoint_weights_pair<K>(p, base, s_lo + msb, s_lo + msb2, srec, sgid, fx, fy0, fy1,
-                                    lane, dfeat);
+            adjoint_weights_pair<K, NP>(p, base, s_lo + msb, s_lo + msb2, srec, sgid, fx, fy, lane,
+                                        dfeat);
           continue;
         }
         const int jj = s_lo + msb;
         const int idx = base + jj;
-        float x[NV];
+        float x[NREAL];
 #pragma unroll
-        for (int v = 0; v < NV; ++v) x[v] = 0.f;
+        for (int v = 0; v < NREAL; ++v) x[v] = 0.f;
         const float4 v0 = srec[jj];
         const float4 v1 = srec[kBatch + jj];
-        const float dx = v0.x - fx, dy0 = v0.y - fy0, dy1 = v0.y - fy1;
-        const float m0 = fminf(0.f, half_form(v0.z, v0.w, v1.x, dx, dy0));
-        const float m1 = fminf(0.f, half_form(v0.z, v0.w, v1.x, dx, dy1));
-        bool hit = adjoint_pixel<K, GEOM, DTAU>(p[0], idx, m0, v0, v1, dx, dy0, srec, jj, x);
-        hit |= adjoint_pixel<K, GEOM, DTAU>(p[1], idx, m1, v0, v1, dx, dy1, srec, jj, x);
+        const float dx = v0.x - fx;
+        float f[K];
+        if (GEOM) load_feats<K>(srec, jj, v1.w, f);
+        bool hit = false;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          const float dy = v0.y - fy[q];
+          const float m = fminf(0.f, half_form(v0.z, v0.w, v1.x, dx, dy));
+          hit |= adjoint_pixel<K, GEOM>(p[q], idx, m, v1, dx, dy, f, x);
+        }
+        if constexpr (GEOM) finish_geom<K>(v0, v1, x);
         const unsigned cm = __ballot_sync(0xffffffffu, hit);
         if (!cm) continue;
         const int64_t g = sgid[jj];
         if (__popc(cm) == 1) {
           if (hit) {
 #pragma unroll
-            for (int k = 0; k < K; ++k) atomicAdd(dfeat + g * K + k, x[k]);
-            if (GEOM) {
-              atomicAdd(dalpha + g, x[K]);
-              atomicAdd(du + 2 * g, x[K + 1]);
-              atomicAdd(du + 2 * g + 1, x[K + 2]);
-              atomicAdd(dconic + 3 * g, x[K + 3]);
-              atomicAdd(dconic + 3 * g + 1, x[K + 4]);
-              atomicAdd(dconic + 3 * g + 2, x[K + 5]);
-            }
+            for (int v = 0; v < NREAL; ++v)
+              atomicAdd(grad_slot<K>(v, g, dfeat, dalpha, du, dconic), x[v]);
           }
           continue;
         }
         int vidx;
         bool owner;
-        const float tot = warp_transpose_sum<NV>(x, lane, &vidx, &owner);
-        if (owner && vidx < NREAL) {
-          float* dst;
-          if (vidx < K)
-            dst = dfeat + g * K + vidx;
-          else if (vidx == K)
-            dst = dalpha + g;
-          else if (vidx < K + 3)
-            dst = du + 2 * g + (vidx - K - 1);
-          else
-            dst = dconic + 3 * g + (vidx - K - 3);
-          atomicAdd(dst, tot);
-        }
+        const float tot = warp_spread_sum<NREAL, 16>(x, lane, &vidx, &owner);
+        if (owner)
+          atomicAdd(grad_slot<K>(vidx, g, dfeat, dalpha, du, dconic), tot);
       }
     }
   }
 }
+
+// Up to this many tiles (4 blocks per SM) a warp is alone on its scheduler or
+// nearly so, and the time is the longest tile's chain of records: with one
+// pixel per lane it is shorter (256 tiles, 20k Gaussians: 91 -> 63 us).  On
+// larger images the instructions count, 1.35x as many (1M Gaussians, 8160
+// tiles: 0.315 against 0.429 ms).
+constexpr int kOnePixelTiles = 592;
 
 template <int K>
 static void draw_bwd_k(int tiles, int H, int W, int gx, const int2* rg, const int32_t* gsid,
                        const float4* rec, const int32_t* order, const int32_t* contrib,
                        const float* ft, const float* dout, const float* dtau, float* dfeat,
                        float* dalpha, float* du, float* dq, cudaStream_t st) {
-  const bool geom = dalpha != nullptr;
-  auto kern = (geom && dtau) ? k_draw_backward<K, true, true>
-              : geom         ? k_draw_backward<K, true, false>
-                             : k_draw_backward<K, false, false>;
-  launch_pdl(kern, dim3(tiles), dim3(kAdjThreads), 0, st, H, W, gx, rg, gsid, rec, order, contrib,
-             ft, dout, dtau, dfeat, dalpha, du, dq);
+  const bool one = tiles <= kOnePixelTiles;
+  auto kern = one ? (dalpha ? k_draw_backward<K, true, 1> : k_draw_backward<K, false, 1>)
+                  : (dalpha ? k_draw_backward<K, true, 2> : k_draw_backward<K, false, 2>);
+  launch_pdl(kern, dim3(tiles), dim3(kTilePixels / (one ? 1 : 2)), 0, st, H, W, gx, rg, gsid, rec,
+             order, contrib, ft, dout, dtau, dfeat, dalpha, du, dq);
 }
 
 int launch_draw_backward(int64_t n, int H, int W, int channels, const int32_t* ranges,
