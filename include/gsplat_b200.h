@@ -303,6 +303,12 @@ int gsb_palette_geo_loss(int chroma_count, int height, int width, const float* l
                          float lambda_pos, float* target_weights, float* loss, float* dlayer,
                          float* dchroma, void* stream);
 
+/* out0[i] = in0[i] * factor[0], out1[i] = in1[i] * factor[0] (device scalar): the
+ * losses' gradients times the incoming gradient, one launch.  Either array may
+ * be empty; in and out must not overlap. */
+int gsb_scale_gradients(int64_t n0, const float* in0, float* out0, int64_t n1,
+                        const float* in1, float* out1, const float* factor, void* stream);
+
 /* The differentiation workload's loss, one launch (plus a one-block init): the
  * colour image img_c = sum_k palette[k][c] layer_k and
  *   loss[0] = (1 - lambda_ssim) loss[1] + lambda_ssim (1 - loss[2]) + loss[3],

@@ -424,6 +424,15 @@ GSB_API int gsb_palette_l1(int K, int height, int width, const float* layer,
                            ST(stream));
 }
 
+GSB_API int gsb_scale_gradients(int64_t n0, const float* in0, float* out0, int64_t n1,
+                                const float* in1, float* out1, const float* factor,
+                                void* stream) {
+  GSB_CHECK_ARG(n0 >= 0 && n1 >= 0 && factor, "scale_gradients: bad size or null factor");
+  GSB_CHECK_ARG((n0 == 0 || (in0 && out0)) && (n1 == 0 || (in1 && out1)),
+                "scale_gradients: null pointer");
+  return launch_scale_gradients(n0, in0, out0, n1, in1, out1, factor, ST(stream));
+}
+
 GSB_API int gsb_palette_l1_ssim(int K, int height, int width, const float* layer,
                                 const float* palette, const float* target, float lambda_ssim,
                                 float lambda_pos, float data_range, float* image, float* loss,
@@ -545,13 +554,14 @@ static int render_backward(int64_t n, const gsb_camera* cam, const float* pws, c
   if ((rc = check_params("render_backward", n, params))) return rc;
   GSB_CHECK_ARG(state && ranges && contrib && final_tau && dloss_dout,
                 "render_backward: null pointer");
-  GSB_CHECK_ARG(n == 0 || (scratch && dw0 && pws && rots && scales && alphas),
-                "render_backward: null input/output");
+  GSB_CHECK_ARG(n == 0 || (scratch && dw0 && pws), "render_backward: null input/output");
   GSB_CHECK_ARG(params->mode == GSB_WEIGHTS_FULL || n == 0 || (dA && dB),
                 "render_backward: null low-rank gradient outputs");
   const bool geom = dpws || drots || dscales || dalphas;
   GSB_CHECK_ARG(!geom || (dpws && drots && dscales && dalphas),
                 "render_backward: pass all of dpws, drots, dscales, dalphas or none");
+  GSB_CHECK_ARG(n == 0 || !geom || (rots && scales && alphas),
+                "render_backward: null geometry input");
   GSB_CHECK_ARG(!params->palette, "render_backward: the palette-colour render has no adjoint here");
   const int K = params->K;
   const SplatState s = carve_state((void*)state, n, K, cam->height, cam->width);

@@ -35,6 +35,9 @@ int lowrank_status(uint32_t* out, bool clear, cudaStream_t st);
 const uint32_t* lowrank_status_word();
 
 // loss.cu
+// out = in * *factor for up to two arrays, one launch.
+int launch_scale_gradients(int64_t n0, const float* in0, float* out0, int64_t n1,
+                           const float* in1, float* out1, const float* factor, cudaStream_t st);
 int launch_palette_l1(int K, int H, int W, const float* layer, const float* palette,
                       const float* target, float* image, float* loss, float* dlayer, float* dpal,
                       cudaStream_t st);

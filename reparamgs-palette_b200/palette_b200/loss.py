@@ -28,6 +28,22 @@ import torch
 from gsplatcu import _lib
 
 
+def _times(g, first, second):
+    """(first * g, second * g) for the incoming gradient `g`, a device scalar,
+    in one launch; either may be None.  Under create_graph the products are
+    torch's, so that they can be differentiated again."""
+    if first is None or torch.is_grad_enabled() or not (
+            g.is_cuda and g.dtype == torch.float32 and g.device == first.device):
+        return (None if first is None else first * g, None if second is None else second * g)
+    a = torch.empty_like(first)
+    b = None if second is None else torch.empty_like(second)
+    with _lib.on_device(first.device):
+        _lib.call("loss.backward", "gsb_scale_gradients", first.numel(), _lib.ptr(first),
+                  _lib.ptr(a), 0 if b is None else second.numel(), _lib.ptr(second), _lib.ptr(b),
+                  _lib.ptr(g), _lib.stream_of(first))
+    return a, b
+
+
 class PaletteL1Loss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, layer, palette, target):
@@ -51,8 +67,7 @@ class PaletteL1Loss(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        dlayer, dpal = ctx.saved_tensors
-        return dlayer * g, dpal * g, None
+        return (*_times(g, *ctx.saved_tensors), None)
 
 
 def palette_l1_loss(layer, palette, target):
@@ -101,8 +116,7 @@ class PaletteGeoLoss(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        dlayer, dchroma = ctx.saved_tensors
-        return dlayer * g, dchroma * g, None, None, None, None
+        return (*_times(g, *ctx.saved_tensors), None, None, None, None)
 
 
 def palette_geo_loss(layer, chroma, target, clamp=False, lambda_pos=0.5, kind="mse"):
@@ -168,10 +182,7 @@ class PaletteL1SsimLoss(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        dlayer, dpal = ctx.saved_tensors
-        g = g[0]
-        return (None if dlayer is None else dlayer * g, None if dpal is None else dpal * g,
-                None, None, None, None)
+        return (*_times(g[0], *ctx.saved_tensors), None, None, None, None)
 
 
 def palette_l1_ssim_loss(layer, palette, target, lambda_ssim=0.2, lambda_pos=0.5,
