@@ -173,17 +173,6 @@ __device__ __forceinline__ void bf16_rows_to_float(const __nv_bfloat16* src, flo
   for (int e = threadIdx.x; e < count; e += blockDim.x) dst[e] = __bfloat162float(src[e]);
 }
 
-// Full-SH rows are 16K floats long, a multiple of 16: written one row per
-// thread, the 32 lanes of a warp would hit 2 (or 1) of the 32 shared-memory
-// banks.  The adjoint therefore builds its SH-gradient rows at an odd stride
-// and packs them before storing them.
-template <int W>
-struct PadRows {
-  static constexpr bool kPad = W > 1 && W % 2 == 0;
-  static constexpr int kStride = kPad ? W + 1 : W;
-  static constexpr int kExtra = kPad ? W + 1 : 0;  // extra floats per thread
-};
-
 // Palette weights of one Gaussian from its staged parameter rows.
 template <int MODE, int K, int P, int Q, int R>
 __device__ __forceinline__ void weights_of(const float* w0, const float* wa, const float* wb,
@@ -368,32 +357,45 @@ __global__ void __launch_bounds__(kFuseThreads)
 // Shared-memory plan of the backward kernel: only the rows it reads are
 // staged -- the centre (view direction), the weight gradients from the
 // compositing adjoint, the low-rank factors (their gradients need each
-// other), and with GEOM also rotation, scale, opacity and the SH
-// coefficients (the view-direction term); the parameter gradients are
-// assembled in shared memory and written back as contiguous spans.
-template <int MODE, int K, int P, int Q, int R, bool GEOM>
+// other), and with GEOM also rotation, scale and the SH coefficients (the
+// view-direction term).  Low-rank gradients are assembled in shared memory and
+// written back as contiguous spans; full-SH gradients are formed while they are
+// written.  What bounds it: HBM (full SH, GEOM: 760 B per Gaussian).  At 500k
+// Gaussians, K = 5, full adjoint: 0.204 -> 0.086 ms (58 us at the copy rate) --
+// SH rows at a conflict-free stride, no gradient rows in shared memory (65 -> 31
+// KB per block), one product sum per SH band, and the geometry chain in FP64
+// through matrix products instead of Jacobian tables (166 -> 100 registers).
+template <int MODE, int K, int P, int Q, int R, typename T, bool GEOM>
 struct BwdPlan {
   using WS = WRows<MODE, K, P, Q, R>;
-  static constexpr bool kW0 = GEOM && MODE == GSB_WEIGHTS_FULL;  // shs needed
-  static constexpr bool kAB = MODE != GSB_WEIGHTS_FULL;
+  static constexpr bool kFull = MODE == GSB_WEIGHTS_FULL;
+  static constexpr bool kW0 = GEOM && kFull;  // shs needed
+  static constexpr bool kAB = !kFull;
+  // Full-SH rows are staged in their storage type, one row per thread, at a
+  // stride of an odd number of 16-byte units: a thread reading its row 16 bytes
+  // at a time shares no bank with its neighbours.
+  static constexpr int kRowUnits = WS::W0 * (int)sizeof(T) / 16;
+  static constexpr int kRowFloats = 4 * (kRowUnits | 1);
   // input regions, in floats per Gaussian (offset = prefix * blockDim)
-  static constexpr int P_ = 3, G_ = K, Q_ = GEOM ? 4 : 0, S_ = GEOM ? 3 : 0, W0_ = kW0 ? WS::W0 : 0,
-                       A_ = kAB ? WS::WA : 0, B_ = kAB ? WS::WB : 0;
-  static constexpr int o_p = 0, o_g = o_p + P_, o_q = o_g + G_, o_s = o_q + Q_, o_w0 = o_s + S_,
-                       o_a = o_w0 + W0_, o_b = o_a + A_, in_floats = o_b + B_;
-  // output regions: d_w0, d_wa, d_wb
-  static constexpr int out_floats = WS::W0 + WS::WA + WS::WB;
+  static constexpr int P_ = 3, G_ = K, Q_ = GEOM ? 4 : 0, S_ = GEOM ? 3 : 0,
+                       W0_ = kW0 ? kRowFloats : 0, A_ = kAB ? WS::WA : 0, B_ = kAB ? WS::WB : 0;
+  static constexpr int o_w0 = 0, o_p = o_w0 + W0_, o_g = o_p + P_, o_q = o_g + G_, o_s = o_q + Q_,
+                       o_a = o_s + S_, o_b = o_a + A_, in_floats = o_b + B_;
+  // output regions: low-rank d_w0, d_wa, d_wb; full SH the basis Y only, since
+  // dL/dshs[l K + k] = Y[l] dL/dw[k] is formed where it is written
+  static constexpr int kBasis = 17;  // 16 values at an odd stride
+  static constexpr int out_floats = kFull ? kBasis : WS::W0 + WS::WA + WS::WB;
   static constexpr int o_dw0 = in_floats, o_dwa = o_dw0 + WS::W0, o_dwb = o_dwa + WS::WA;
-  static constexpr int floats = in_floats + out_floats;
-};
-
-// Raw BF16 rows of the backward's staged colour parameters (bulk-copied,
-// then converted into their float areas), in floats per thread.
-template <int MODE, int K, int P, int Q, int R, bool GEOM, typename T>
-struct BwdRaw {
-  using BP = BwdPlan<MODE, K, P, Q, R, GEOM>;
-  static constexpr int kHalfs = sizeof(T) == 2 ? BP::W0_ + BP::A_ + BP::B_ : 0;
-  static constexpr int kFloats = (kHalfs + 1) / 2;
+  static constexpr int o_y = in_floats;
+  // low-rank d_w0 rows of an even length are built at an odd stride past the
+  // plan's regions and packed before they are stored
+  static constexpr bool kPad = !kFull && WS::W0 > 1 && WS::W0 % 2 == 0;
+  static constexpr int kPadStride = kPad ? WS::W0 + 1 : WS::W0;
+  // raw BF16 low-rank factors, bulk-copied, then converted into their float areas
+  static constexpr int kRawFloats = sizeof(T) == 2 ? (A_ + B_ + 1) / 2 : 0;
+  static constexpr int o_pad = in_floats + out_floats;
+  static constexpr int o_raw = o_pad + (kPad ? WS::W0 + 1 : 0);
+  static constexpr int floats = o_raw + kRawFloats;
 };
 
 // Stages the block's input rows.  With `acc` (gradients added to what the
@@ -409,31 +411,34 @@ __device__ __forceinline__ int stage_backward(int64_t n, int64_t row0, const flo
                                               const float* g_feat, bool acc, const float* d_w0,
                                               const float* d_wa, const float* d_wb, float* sm,
                                               float* raw, uint64_t* bar) {
-  using BP = BwdPlan<MODE, K, P, Q, R, GEOM>;
+  using BP = BwdPlan<MODE, K, P, Q, R, T, GEOM>;
   using WS = WRows<MODE, K, P, Q, R>;
   const int nt = blockDim.x;
   const bool full = row0 + nt <= n;
   bool bulk = full && aligned16(pws + row0 * 3) && aligned16(g_feat + row0 * K);
   if (GEOM) bulk = bulk && aligned16(rots + row0 * 4) && aligned16(scales + row0 * 3);
-  if (BP::kW0)
-    bulk = bulk && aligned16(w0 + row0 * WS::W0) && (nt * WS::W0 * sizeof(T)) % 16 == 0;
+  if (BP::kW0) bulk = bulk && aligned16(w0 + row0 * WS::W0);
   if (BP::kAB)
     bulk = bulk && aligned16(wa + row0 * WS::WA) && aligned16(wb + row0 * WS::WB) &&
            (nt * WS::WA * sizeof(T)) % 16 == 0 && (nt * WS::WB * sizeof(T)) % 16 == 0;
-  const bool raw16 = bulk && sizeof(T) == 2;
-  bool pre = bulk && acc && aligned16(d_w0 + row0 * WS::W0) && (nt * WS::W0 * 4) % 16 == 0;
-  if (MODE != GSB_WEIGHTS_FULL)
-    pre = pre && aligned16(d_wa + row0 * WS::WA) && aligned16(d_wb + row0 * WS::WB) &&
-          (nt * WS::WA * 4) % 16 == 0 && (nt * WS::WB * 4) % 16 == 0;
+  const bool raw16 = bulk && BP::kAB && sizeof(T) == 2;
+  const bool pre = !BP::kFull && bulk && acc && aligned16(d_w0 + row0 * WS::W0) &&
+                   (nt * WS::W0 * 4) % 16 == 0 && aligned16(d_wa + row0 * WS::WA) &&
+                   aligned16(d_wb + row0 * WS::WB) && (nt * WS::WA * 4) % 16 == 0 &&
+                   (nt * WS::WB * 4) % 16 == 0;
   if (bulk && threadIdx.x == 0) {
     mbar_init(bar, 1);
-    mbar_arrive_expect_tx(bar, (uint32_t)(nt * (BP::P_ + BP::G_ + BP::Q_ + BP::S_) * 4 +
-                                          nt * (BP::W0_ + BP::A_ + BP::B_) * sizeof(T) +
-                                          (pre ? nt * BP::out_floats * 4 : 0)));
+    mbar_arrive_expect_tx(
+        bar, (uint32_t)(nt * (BP::P_ + BP::G_ + BP::Q_ + BP::S_) * 4 +
+                        nt * ((BP::kW0 ? WS::W0 : 0) + BP::A_ + BP::B_) * sizeof(T) +
+                        (pre ? nt * BP::out_floats * 4 : 0)));
   }
-  if (pre && threadIdx.x == 0) {
-    bulk_load(sm + nt * BP::o_dw0, d_w0 + row0 * WS::W0, (uint32_t)(nt * WS::W0 * 4), bar);
-    if constexpr (MODE != GSB_WEIGHTS_FULL) {
+  if constexpr (BP::kW0) {
+    if (bulk) __syncthreads();  // the barrier is initialised before any thread's copy
+  }
+  if constexpr (!BP::kFull) {
+    if (pre && threadIdx.x == 0) {
+      bulk_load(sm + nt * BP::o_dw0, d_w0 + row0 * WS::W0, (uint32_t)(nt * WS::W0 * 4), bar);
       bulk_load(sm + nt * BP::o_dwa, d_wa + row0 * WS::WA, (uint32_t)(nt * WS::WA * 4), bar);
       bulk_load(sm + nt * BP::o_dwb, d_wb + row0 * WS::WB, (uint32_t)(nt * WS::WB * 4), bar);
     }
@@ -444,22 +449,28 @@ __device__ __forceinline__ int stage_backward(int64_t n, int64_t row0, const flo
     stage_rows<4>(rots, row0, n, sm + nt * BP::o_q, bulk, bar);
     stage_rows<3>(scales, row0, n, sm + nt * BP::o_s, bulk, bar);
   }
-  if (raw16) {
-    if (threadIdx.x == 0) {
-      char* r = (char*)raw;
-      if constexpr (BP::kW0) {
-        bulk_load(r, w0 + row0 * WS::W0, (uint32_t)(nt * WS::W0 * 2), bar);
-        r += nt * WS::W0 * 2;
-      }
-      if constexpr (BP::kAB) {
-        bulk_load(r, wa + row0 * WS::WA, (uint32_t)(nt * WS::WA * 2), bar);
-        r += nt * WS::WA * 2;
-        bulk_load(r, wb + row0 * WS::WB, (uint32_t)(nt * WS::WB * 2), bar);
+  if constexpr (BP::kW0) {
+    T* rows = reinterpret_cast<T*>(sm + nt * BP::o_w0);
+    constexpr int stride = BP::kRowFloats * 4 / (int)sizeof(T);
+    if (bulk) {
+      bulk_load(rows + threadIdx.x * stride, w0 + (row0 + threadIdx.x) * WS::W0,
+                (uint32_t)(WS::W0 * sizeof(T)), bar);
+    } else {
+      const int64_t count = min((int64_t)nt, n - row0) * WS::W0;
+      for (int e = threadIdx.x; e < count; e += nt) {
+        const int r = e / WS::W0, c = e - r * WS::W0;
+        rows[r * stride + c] = w0[row0 * WS::W0 + e];
       }
     }
-  } else {
-    if constexpr (BP::kW0) stage_rows<WS::W0>(w0, row0, n, sm + nt * BP::o_w0, bulk, bar);
-    if constexpr (BP::kAB) {
+  }
+  if constexpr (BP::kAB) {
+    if (raw16) {
+      if (threadIdx.x == 0) {
+        bulk_load(raw, wa + row0 * WS::WA, (uint32_t)(nt * WS::WA * 2), bar);
+        bulk_load((char*)raw + nt * WS::WA * 2, wb + row0 * WS::WB, (uint32_t)(nt * WS::WB * 2),
+                  bar);
+      }
+    } else {
       stage_rows<WS::WA>(wa, row0, n, sm + nt * BP::o_a, bulk, bar);
       stage_rows<WS::WB>(wb, row0, n, sm + nt * BP::o_b, bulk, bar);
     }
@@ -470,17 +481,11 @@ __device__ __forceinline__ int stage_backward(int64_t n, int64_t row0, const flo
     mbar_wait(bar, 0);  // bounded second wait for copies still in flight
     return 0;
   }
-  if constexpr (sizeof(T) == 2) {  // raw BF16 rows -> their float areas
+  if constexpr (BP::kAB && sizeof(T) == 2) {  // raw BF16 factors -> their float areas
     if (raw16) {
       const __nv_bfloat16* r = (const __nv_bfloat16*)raw;
-      if constexpr (BP::kW0) {
-        bf16_rows_to_float(r, sm + nt * BP::o_w0, nt * WS::W0);
-        r += nt * WS::W0;
-      }
-      if constexpr (BP::kAB) {
-        bf16_rows_to_float(r, sm + nt * BP::o_a, nt * WS::WA);
-        bf16_rows_to_float(r + nt * WS::WA, sm + nt * BP::o_b, nt * WS::WB);
-      }
+      bf16_rows_to_float(r, sm + nt * BP::o_a, nt * WS::WA);
+      bf16_rows_to_float(r + nt * WS::WA, sm + nt * BP::o_b, nt * WS::WB);
     }
     __syncthreads();
   }
@@ -544,23 +549,20 @@ __global__ void __launch_bounds__(kFuseThreads)
                           float* __restrict__ d_wa, float* __restrict__ d_wb, bool acc) {
   pdl_wait();
   using WS = WRows<MODE, K, P, Q, R>;
-  using BP = BwdPlan<MODE, K, P, Q, R, GEOM>;
+  using BP = BwdPlan<MODE, K, P, Q, R, T, GEOM>;
   constexpr int L = WS::L;
   extern __shared__ __align__(16) float sm[];
   __shared__ __align__(8) uint64_t bar;
   const int nt = blockDim.x, t = threadIdx.x;
   const int64_t row0 = (int64_t)blockIdx.x * nt;
-  float* raw = sm + nt * (BP::floats + PadRows<WS::W0>::kExtra);
   const int staged = stage_backward<MODE, K, P, Q, R, GEOM, T>(
-      n, row0, pws, rots, scales, w0, wa, wb, g_feat, acc, d_w0, d_wa, d_wb, sm, raw, &bar);
+      n, row0, pws, rots, scales, w0, wa, wb, g_feat, acc, d_w0, d_wa, d_wb, sm,
+      sm + nt * BP::o_raw, &bar);
   if (!staged) return;
   const bool pre = staged == 2;  // the outputs' rows are in the gradient area: add to them
   const auto put = [pre](float* d, float v) { *d = pre ? *d + v : v; };
   const int64_t i = row0 + t;
-  // full-SH gradient rows are built at an odd stride past the plan's regions
-  // (see PadRows) and packed contiguously before they are stored
-  using PR = PadRows<WS::W0>;
-  float* o_w0 = PR::kPad ? sm + nt * BP::floats + t * PR::kStride : sm + nt * BP::o_dw0 + t * WS::W0;
+  float* o_w0 = BP::kPad ? sm + nt * BP::o_pad + t * BP::kPadStride : sm + nt * BP::o_dw0 + t * WS::W0;
   float* o_wa = sm + nt * BP::o_dwa + t * WS::WA;
   float* o_wb = sm + nt * BP::o_dwb + t * WS::WB;
   if (i < n) {
@@ -606,71 +608,103 @@ __global__ void __launch_bounds__(kFuseThreads)
           double dc2[3];
 #pragma unroll
           for (int j = 0; j < 3; ++j) dc2[j] = gq[0] * Ji[j] + gq[1] * Ji[3 + j] + gq[2] * Ji[6 + j];
-          double c3d[6], M2d[6], Rd[9];
+          // cov2d = M S M^T with M = J Rcw: dL/dS = M^T G M, dL/dM = 2 G M S,
+          // G the symmetric gradient of cov2d
+          const double g01 = 0.5 * dc2[1];
+          double Md[6], Rd[9], GM[6];
 #pragma unroll
-          for (int u = 0; u < 6; ++u) { c3d[u] = cov3[u]; M2d[u] = M2[u]; }
+          for (int u = 0; u < 6; ++u) Md[u] = M2[u];
 #pragma unroll
           for (int u = 0; u < 9; ++u) Rd[u] = cr.R[u];
-          double d3[18], dpc_m[9];
-          cov2d_jacobians<double>(c3d, M2d, Rd, xy[0], xy[1], p.z, cam.fx, cam.fy, d3, dpc_m);
-          double dS[6];
 #pragma unroll
-          for (int u = 0; u < 6; ++u)
-            dS[u] = dc2[0] * d3[u] + dc2[1] * d3[6 + u] + dc2[2] * d3[12 + u];
-          double dpc[3];
+          for (int j = 0; j < 3; ++j) {
+            GM[j] = dc2[0] * Md[j] + g01 * Md[3 + j];
+            GM[3 + j] = g01 * Md[j] + dc2[2] * Md[3 + j];
+          }
+          double dS[6];  // 00 01 02 11 12 22 of the symmetric gradient
 #pragma unroll
-          for (int j = 0; j < 3; ++j)
-            dpc[j] = dc2[0] * dpc_m[j] + dc2[1] * dpc_m[3 + j] + dc2[2] * dpc_m[6 + j];
+          for (int r = 0, u = 0; r < 3; ++r)
+#pragma unroll
+            for (int j = r; j < 3; ++j, ++u) dS[u] = Md[r] * GM[j] + Md[3 + r] * GM[3 + j];
+          // dL/dM, then M's dependence on the camera-space centre
+          const double c00 = cov3[0], c01 = cov3[1], c02 = cov3[2], c11 = cov3[3], c12 = cov3[4],
+                       c22 = cov3[5];
+          double t2[2], tz[2];  // row r of dL/dM against Rcw's rows 2 and r
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const double g0 = GM[3 * r], g1 = GM[3 * r + 1], g2 = GM[3 * r + 2];
+            const double m0 = 2.0 * (g0 * c00 + g1 * c01 + g2 * c02);
+            const double m1 = 2.0 * (g0 * c01 + g1 * c11 + g2 * c12);
+            const double m2 = 2.0 * (g0 * c02 + g1 * c12 + g2 * c22);
+            t2[r] = m0 * Rd[6] + m1 * Rd[7] + m2 * Rd[8];
+            tz[r] = m0 * Rd[3 * r] + m1 * Rd[3 * r + 1] + m2 * Rd[3 * r + 2];
+          }
           const double zi = 1.0 / p.z, zi2 = zi * zi;
-          dpc[0] += gu[0] * (cam.fx * zi);
-          dpc[1] += gu[1] * (cam.fy * zi);
-          dpc[2] += gu[0] * (-(p.x * (double)cam.fx) * zi2) + gu[1] * (-(p.y * (double)cam.fy) * zi2);
+          const double fxz = cam.fx * zi2, fyz = cam.fy * zi2;
+          double dpc[3];
+          dpc[0] = gu[0] * (cam.fx * zi) - fxz * t2[0];
+          dpc[1] = gu[1] * (cam.fy * zi) - fyz * t2[1];
+          dpc[2] = -gu[0] * (p.x * fxz) - gu[1] * (p.y * fyz) - fxz * tz[0] - fyz * tz[1] +
+                   2.0 * zi * (fxz * xy[0] * t2[0] + fyz * xy[1] * t2[1]);
 #pragma unroll
           for (int j = 0; j < 3; ++j)
             dpw[j] += (float)(Rd[j] * dpc[0] + Rd[3 + j] * dpc[1] + Rd[6 + j] * dpc[2]);
-          double M3d[9], Rqd[9];
+          // Sigma = M3 M3^T, M3 = R(q) diag(s): dL/dM3 = 2 dS M3
+          const double sv[3] = {sc.x, sc.y, sc.z};
+          double dR[9];
 #pragma unroll
-          for (int u = 0; u < 9; ++u) { M3d[u] = M3[u]; Rqd[u] = Rq[u]; }
-          double jq[24], js[18];
-          cov3d_jacobians<double>(q, sc, M3d, Rqd, jq, js);
-          double dqd[4] = {0.0, 0.0, 0.0, 0.0}, dsd[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-          for (int u = 0; u < 6; ++u) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) dqd[j] += dS[u] * jq[4 * u + j];
-#pragma unroll
-            for (int j = 0; j < 3; ++j) dsd[j] += dS[u] * js[3 * u + j];
+          for (int j = 0; j < 3; ++j) {
+            const double m0 = M3[j], m1 = M3[3 + j], m2 = M3[6 + j];
+            const double e0 = 2.0 * (dS[0] * m0 + dS[1] * m1 + dS[2] * m2);
+            const double e1 = 2.0 * (dS[1] * m0 + dS[3] * m1 + dS[4] * m2);
+            const double e2 = 2.0 * (dS[2] * m0 + dS[4] * m1 + dS[5] * m2);
+            ds[j] += (float)(e0 * Rq[j] + e1 * Rq[3 + j] + e2 * Rq[6 + j]);
+            dR[j] = e0 * sv[j];
+            dR[3 + j] = e1 * sv[j];
+            dR[6 + j] = e2 * sv[j];
           }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) dq[j] += (float)dqd[j];
-#pragma unroll
-          for (int j = 0; j < 3; ++j) ds[j] += (float)dsd[j];
+          const double qw = q.x, qx = q.y, qy = q.z, qz = q.w;
+          dq[0] += (float)(2.0 * (qz * (dR[3] - dR[1]) + qy * (dR[2] - dR[6]) +
+                                  qx * (dR[7] - dR[5])));
+          dq[1] += (float)(2.0 * (qy * (dR[1] + dR[3]) + qz * (dR[2] + dR[6]) +
+                                  qw * (dR[7] - dR[5]) - 2.0 * qx * (dR[4] + dR[8])));
+          dq[2] += (float)(2.0 * (qx * (dR[1] + dR[3]) + qw * (dR[2] - dR[6]) +
+                                  qz * (dR[5] + dR[7]) - 2.0 * qy * (dR[0] + dR[8])));
+          dq[3] += (float)(2.0 * (qw * (dR[3] - dR[1]) + qx * (dR[2] + dR[6]) +
+                                  qy * (dR[5] + dR[7]) - 2.0 * qz * (dR[0] + dR[4])));
         }
       }
       sh_basis_grad(dir, L + 1, /*ref_quirk=*/false, G);
     }
     // colour parameters, and (GEOM) the view direction's share of d pws
     float dd[3] = {0.f, 0.f, 0.f};
+    float tl[16];  // sum over k of dL/dw[k] times the coefficient of band l
+    if constexpr (GEOM) {
+#pragma unroll
+      for (int l = 0; l < 16; ++l) tl[l] = 0.f;
+    }
     if constexpr (MODE == GSB_WEIGHTS_FULL) {
-      const float* s_w0 = sm + nt * BP::o_w0 + t * WS::W0;
+      float* y = sm + nt * BP::o_y + t * BP::kBasis;
 #pragma unroll
-      for (int l = 0; l < 16; ++l)
+      for (int l = 0; l < 16; ++l) y[l] = Y[l];
+      if constexpr (GEOM) {
+        constexpr int kPer = 16 / (int)sizeof(T);  // values per 16 bytes
+        const uint4* row = reinterpret_cast<const uint4*>(sm + nt * BP::o_w0 + t * BP::kRowFloats);
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-          o_w0[l * K + k] = gw[k] * Y[l];
-          if constexpr (GEOM) {
-            if (l > 0) {
-              const float cg = gw[k] * s_w0[l * K + k];
-              dd[0] += cg * G[3 * l];
-              dd[1] += cg * G[3 * l + 1];
-              dd[2] += cg * G[3 * l + 2];
-            }
+        for (int u = 0; u < BP::kRowUnits; ++u) {
+          const uint4 v = row[u];
+          const T* e = reinterpret_cast<const T*>(&v);
+#pragma unroll
+          for (int c = 0; c < kPer; ++c) {
+            const int idx = u * kPer + c;
+            tl[idx / K] += gw[idx % K] * as_f32(e[c]);
           }
         }
+      }
     } else {
 #pragma unroll
       for (int k = 0; k < K; ++k) {
-        if constexpr (PR::kPad)
+        if constexpr (BP::kPad)
           o_w0[k] = gw[k] * SH_C0;  // packed (and added) below
         else
           put(o_w0 + k, gw[k] * SH_C0);
@@ -691,12 +725,7 @@ __global__ void __launch_bounds__(kFuseThreads)
             acc[r] += dC * s_wb[r * Q + qq];
             if constexpr (GEOM) coef += s_wa[pp * R + r] * s_wb[r * Q + qq];
           }
-          if constexpr (GEOM) {
-            const float cg = gw[k] * coef;
-            dd[0] += cg * G[3 * (l + 1)];
-            dd[1] += cg * G[3 * (l + 1) + 1];
-            dd[2] += cg * G[3 * (l + 1) + 2];
-          }
+          if constexpr (GEOM) tl[l + 1] += gw[k] * coef;
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) put(o_wa + pp * R + r, acc[r]);
@@ -718,6 +747,13 @@ __global__ void __launch_bounds__(kFuseThreads)
       }
     }
     if constexpr (GEOM) {
+#pragma unroll
+      for (int l = 1; l < 16; ++l)
+        if (l <= L) {
+          dd[0] += tl[l] * G[3 * l];
+          dd[1] += tl[l] * G[3 * l + 1];
+          dd[2] += tl[l] * G[3 * l + 2];
+        }
       float Jd[9];
       dir_jacobian(nd, ninv, Jd);
 #pragma unroll
@@ -731,43 +767,58 @@ __global__ void __launch_bounds__(kFuseThreads)
     }
   }
   // parameter gradients: shared memory -> global, block span by block span;
-  // with `acc` and no preloaded rows (a partial or unaligned block), added to
-  // what the outputs hold by a coalesced read-add-write
-  if (acc && !pre) {
+  // with `acc` and no preloaded rows (full SH, a partial or unaligned block),
+  // added to what the outputs hold by a coalesced read-add-write
+  const int64_t rows = min((int64_t)nt, n - row0);
+  if constexpr (BP::kFull) {
     __syncthreads();
-    const int64_t rows = min((int64_t)nt, n - row0);
-    if constexpr (PR::kPad) {
-      const float* src = sm + nt * BP::floats;
-      add_span<WS::W0>(d_w0, row0, rows, [src](int j) {
-        const int r = j / WS::W0, c = j - r * WS::W0;
-        return src[r * PR::kStride + c];
-      });
+    const float* y = sm + nt * BP::o_y;
+    const float* g = sm + nt * BP::o_g;
+    const auto value = [y, g](int j) {
+      const int r = j / WS::W0, c = j - r * WS::W0, l = c / K;
+      return g[r * K + (c - l * K)] * y[r * BP::kBasis + l];
+    };
+    if (acc) {
+      add_span<WS::W0>(d_w0, row0, rows, value);
+    } else if (aligned16(d_w0 + row0 * WS::W0)) {
+      float4* out = reinterpret_cast<float4*>(d_w0 + row0 * WS::W0);
+      for (int j = t; j < (int)rows * (WS::W0 / 4); j += nt)
+        out[j] = make_float4(value(4 * j), value(4 * j + 1), value(4 * j + 2), value(4 * j + 3));
     } else {
-      add_rows<WS::W0>(d_w0, row0, rows, sm + nt * BP::o_dw0);
+      for (int j = t; j < (int)rows * WS::W0; j += nt) d_w0[row0 * WS::W0 + j] = value(j);
     }
-    if constexpr (MODE != GSB_WEIGHTS_FULL) {
+  } else {
+    if (acc && !pre) {
+      __syncthreads();
+      if constexpr (BP::kPad) {
+        const float* src = sm + nt * BP::o_pad;
+        add_span<WS::W0>(d_w0, row0, rows, [src](int j) {
+          const int r = j / WS::W0, c = j - r * WS::W0;
+          return src[r * BP::kPadStride + c];
+        });
+      } else {
+        add_rows<WS::W0>(d_w0, row0, rows, sm + nt * BP::o_dw0);
+      }
       add_rows<WS::WA>(d_wa, row0, rows, sm + nt * BP::o_dwa);
       add_rows<WS::WB>(d_wb, row0, rows, sm + nt * BP::o_dwb);
+      return;
     }
-    return;
-  }
-  if constexpr (PR::kPad) {
+    if constexpr (BP::kPad) {
+      __syncthreads();
+      float* dst = sm + nt * BP::o_dw0;
+      const float* src = sm + nt * BP::o_pad;
+      for (int e = t; e < nt * WS::W0; e += nt) {
+        const int r = e / WS::W0, c = e - r * WS::W0;
+        dst[e] = pre ? dst[e] + src[r * BP::kPadStride + c] : src[r * BP::kPadStride + c];
+      }
+    }
+    fence_proxy_async_shared();
     __syncthreads();
-    float* dst = sm + nt * BP::o_dw0;
-    const float* src = sm + nt * BP::floats;
-    for (int e = t; e < nt * WS::W0; e += nt) {
-      const int r = e / WS::W0, c = e - r * WS::W0;
-      dst[e] = pre ? dst[e] + src[r * PR::kStride + c] : src[r * PR::kStride + c];
-    }
-  }
-  fence_proxy_async_shared();
-  __syncthreads();
-  write_rows<WS::W0>(d_w0, row0, n, sm + nt * BP::o_dw0);
-  if constexpr (MODE != GSB_WEIGHTS_FULL) {
+    write_rows<WS::W0>(d_w0, row0, n, sm + nt * BP::o_dw0);
     write_rows<WS::WA>(d_wa, row0, n, sm + nt * BP::o_dwa);
     write_rows<WS::WB>(d_wb, row0, n, sm + nt * BP::o_dwb);
+    if (threadIdx.x == 0) bulk_store_drain();
   }
-  if (threadIdx.x == 0) bulk_store_drain();
 }
 
 // ------------------------------------------------------------ dispatch
@@ -798,11 +849,8 @@ static int launch_fused(const FusedArgs& f, bool backward, cudaStream_t st) {
   const bool geom = f.g_u != nullptr;
   auto kern = geom ? k_render_backward_pre<MODE, K, P, Q, R, T, true>
                    : k_render_backward_pre<MODE, K, P, Q, R, T, false>;
-  const int bsmem = ((geom ? BwdPlan<MODE, K, P, Q, R, true>::floats +
-                                 BwdRaw<MODE, K, P, Q, R, true, T>::kFloats
-                           : BwdPlan<MODE, K, P, Q, R, false>::floats +
-                                 BwdRaw<MODE, K, P, Q, R, false, T>::kFloats) +
-                     PadRows<WS::W0>::kExtra) *
+  const int bsmem = (geom ? BwdPlan<MODE, K, P, Q, R, T, true>::floats
+                          : BwdPlan<MODE, K, P, Q, R, T, false>::floats) *
                     kFuseThreads * 4;
   if ((rc = set_smem(kern, bsmem))) return rc;
   launch_pdl(kern, dim3(grid), dim3(kFuseThreads), bsmem, st, f.n, f.cam, f.pws, f.rots,

@@ -339,9 +339,7 @@ __device__ __forceinline__ void lowrank_weights(const S* dc, const S* a, const S
 }
 
 // ------------------------------------------------------------ Jacobians
-// Computed in the scalar type T: float for the operators' Jacobian outputs,
-// double in the adjoint's geometry chain (in FP32 that chain's rotation and
-// scale gradients lost up to 3e-4 relative to rounding).
+// For the operators' Jacobian outputs.
 // d Sigma_(rc) / d q_j and / d s_j for Sigma = M M^T, M = R(q) diag(s).
 template <typename T>
 __device__ __forceinline__ void cov3d_jacobians(float4 q, float3 s, const T* M, const T* R,
