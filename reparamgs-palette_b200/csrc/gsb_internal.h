@@ -108,6 +108,19 @@ int launch_sort_capacity(const SortPlan& p, int64_t n, int H, int W, const Splat
                          void* ws, int32_t* gsid_out, int32_t* ranges_out, uint32_t* status,
                          cudaStream_t st);
 
+// tile_lists.cu -- the same lists and ranges as launch_sort[_capacity], by a depth
+// sort of the Gaussians and a stable fill of the tiles (mdev null: p.M is exact).
+struct ListPlan {
+  bool ok;  // the sizes are within this path's limits
+  int64_t n, M, tiles, sort_blocks, groups;
+  int gx, gy, dkey_bits, passes, digit_bits, chunks, pitch, bands, band_rows, count_bands, count_rows;
+  size_t off_keys[2], off_vals[2], off_rects, off_hist, off_digit_tot, off_groups, off_bounds,
+      off_counts, off_tile_tot, bytes_total;
+};
+ListPlan make_list_plan(int64_t n, int H, int W, int64_t M, uint32_t max_dkey);
+int launch_tile_lists(const ListPlan& p, const SplatState& s, void* ws, int32_t* gsid_out,
+                      int32_t* ranges_out, const uint32_t* mdev, cudaStream_t st);
+
 // raster.cu, raster_backward.cu
 // Launch order of the compositing tiles, longest list first.
 int launch_tile_order(const int2* ranges, int tiles, int32_t* order, cudaStream_t st);
