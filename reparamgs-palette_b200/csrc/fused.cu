@@ -36,12 +36,27 @@ struct WRows {
   static constexpr int WA = MODE == GSB_WEIGHTS_FULL ? 0 : P * R;
   static constexpr int WB = MODE == GSB_WEIGHTS_FULL ? 0 : R * Q;
   static constexpr int L = MODE == GSB_WEIGHTS_FULL ? 15 : P * Q / K;
-  static constexpr int IN = 3 + 4 + 3 + 1 + W0 + WA + WB;  // staged floats per Gaussian
-  // The forward stages full-SH rows (16K floats, a multiple of 16) at a stride
-  // of an odd number of float4s, so that one thread per row reading float4s
-  // touches distinct shared-memory banks; other rows stay contiguous.
-  static constexpr int W0S = MODE == GSB_WEIGHTS_FULL ? 4 * ((W0 / 4) | 1) : W0;
-  static constexpr int INS = 3 + 4 + 3 + 1 + W0S + WA + WB;  // forward staged floats
+};
+
+// Shared memory of the forward, in floats per Gaussian.  Full-SH rows are staged
+// in their storage type at a stride of an odd number of 16-byte units, so that
+// one thread per row reading 16 bytes at a time touches distinct banks; other
+// rows stay contiguous.  `kRawFloats`: bulk-copied low-rank BF16 rows, read as
+// they are (their float areas serve the unaligned case).  What bounds it: HBM,
+// given enough blocks per SM to keep loads in flight.  3M Gaussians, K = 5, BF16
+// full SH: 0.259 -> 0.163 ms (0.13 at the copy rate) without the raw copy of the
+// rows and its conversion pass (35 -> 14 KB per block, 6 -> 16 blocks per SM); 1M,
+// rank 3: 0.067 ms at 5.6 TB/s.
+template <int MODE, int K, int P, int Q, int R, typename T>
+struct FwdPlan {
+  using WS = WRows<MODE, K, P, Q, R>;
+  static constexpr int kRowUnits = WS::W0 * (int)sizeof(T) / 16;
+  static constexpr int kW0 = MODE == GSB_WEIGHTS_FULL ? 4 * (kRowUnits | 1) : WS::W0;
+  static constexpr int kStride = kW0 * 4 / (int)sizeof(T);  // full-SH row, in elements
+  static constexpr int kStaged = 3 + 4 + 3 + 1 + kW0 + WS::WA + WS::WB;
+  static constexpr int kRawFloats =
+      sizeof(T) == 2 && MODE != GSB_WEIGHTS_FULL ? (WS::W0 + WS::WA + WS::WB + 1) / 2 : 0;
+  static constexpr int kFloats = kStaged + kRawFloats;
 };
 
 // Camera: rotation, translation and centre stay in device memory (so a
@@ -65,7 +80,7 @@ __device__ __forceinline__ CamRegs load_cam(const CamArgs& a) {
 
 // Shared-memory regions of one block: the rows of its Gaussians, array by
 // array, back to back.
-template <int MODE, int K, int P, int Q, int R>
+template <int MODE, int K, int P, int Q, int R, typename T>
 struct Staged {
   using WS = WRows<MODE, K, P, Q, R>;
   const float *p, *q, *s, *al, *w0, *wa, *wb;
@@ -76,18 +91,9 @@ struct Staged {
     s = q + nt * 4;
     al = s + nt * 3;
     w0 = al + nt;
-    wa = w0 + nt * WS::W0S;
+    wa = w0 + nt * FwdPlan<MODE, K, P, Q, R, T>::kW0;
     wb = wa + nt * WS::WA;
   }
-};
-
-// Extra shared memory of the forward, in floats per thread, past the staged
-// rows: the raw bulk-copied BF16 colour rows, converted into the float rows.
-template <int MODE, int K, int P, int Q, int R, typename T>
-struct FwdExtra {
-  using WS = WRows<MODE, K, P, Q, R>;
-  static constexpr bool kRawLowrank = sizeof(T) == 2 && MODE != GSB_WEIGHTS_FULL;
-  static constexpr int kRawFloats = sizeof(T) == 2 ? (WS::W0 + WS::WA + WS::WB + 1) / 2 : 0;
 };
 
 // How the block's colour-parameter rows ended up in shared memory.
@@ -95,10 +101,9 @@ enum StageResult { kStageFailed = 0, kStagedFloat = 1, kStagedRawBf16 = 2 };
 
 // Stage one block's parameter rows (pws, rots, scales, alphas, colour
 // parameters) into shared memory, by bulk copies when the block is full and
-// every span is 16-byte aligned.  FP32 rows land in their float areas; BF16
-// colour rows are bulk-copied raw (full SH: into the float area of the SH
-// rows; low-rank: into `raw`) and converted by the caller (kStagedRawBf16).
-// Without bulk copies every row is converted to float while staged.
+// every span is 16-byte aligned.  Full-SH rows keep their storage type.  FP32
+// low-rank rows land in their float areas; BF16 ones are bulk-copied into `raw`
+// and read there (kStagedRawBf16), or converted while staged without bulk copies.
 // Returns kStageFailed if a bulk wait expired (the status word is set and the
 // block must not use the staged rows).
 template <int MODE, int K, int P, int Q, int R, typename T>
@@ -107,7 +112,7 @@ __device__ __forceinline__ int stage_params(int64_t n, int64_t row0, const float
                                             const float* alphas, const T* w0, const T* wa,
                                             const T* wb, float* sm, float* raw, uint64_t* bar) {
   using WS = WRows<MODE, K, P, Q, R>;
-  const Staged<MODE, K, P, Q, R> S(sm);
+  const Staged<MODE, K, P, Q, R, T> S(sm);
   const int nt = blockDim.x;
   const bool full = row0 + nt <= n;
   bool bulk = full && aligned16(pws + row0 * 3) && aligned16(rots + row0 * 4) &&
@@ -116,42 +121,40 @@ __device__ __forceinline__ int stage_params(int64_t n, int64_t row0, const float
   if (MODE != GSB_WEIGHTS_FULL)
     bulk = bulk && aligned16(wa + row0 * WS::WA) && aligned16(wb + row0 * WS::WB) &&
            (nt * WS::WA * sizeof(T)) % 16 == 0 && (nt * WS::WB * sizeof(T)) % 16 == 0;
-  const bool raw16 = bulk && sizeof(T) == 2;
+  const bool raw16 = bulk && sizeof(T) == 2 && MODE != GSB_WEIGHTS_FULL;
   if (bulk && threadIdx.x == 0) {
     mbar_init(bar, 1);
     mbar_arrive_expect_tx(
         bar, (uint32_t)(nt * 11 * 4 + nt * (WS::W0 + WS::WA + WS::WB) * sizeof(T)));
   }
-  if constexpr (MODE == GSB_WEIGHTS_FULL && sizeof(T) == 4) {
+  if constexpr (MODE == GSB_WEIGHTS_FULL) {
     if (bulk) __syncthreads();  // the barrier is initialised before any thread's copy
   }
   stage_rows<3>(pws, row0, n, (float*)S.p, bulk, bar);
   stage_rows<4>(rots, row0, n, (float*)S.q, bulk, bar);
   stage_rows<3>(scales, row0, n, (float*)S.s, bulk, bar);
   stage_rows<1>(alphas, row0, n, (float*)S.al, bulk, bar);
-  if (raw16) {
+  if constexpr (MODE == GSB_WEIGHTS_FULL) {
+    constexpr int stride = FwdPlan<MODE, K, P, Q, R, T>::kStride;
+    T* rows = reinterpret_cast<T*>((float*)S.w0);
+    if (bulk) {  // one copy per row
+      bulk_load(rows + threadIdx.x * stride, w0 + (row0 + threadIdx.x) * WS::W0,
+                (uint32_t)(WS::W0 * sizeof(T)), bar);
+    } else {
+      const int64_t count = min((int64_t)nt, n - row0) * WS::W0;
+      for (int e = threadIdx.x; e < count; e += nt) {
+        const int r = e / WS::W0, c = e - r * WS::W0;
+        rows[r * stride + c] = w0[row0 * WS::W0 + e];
+      }
+    }
+  } else if (raw16) {
     if (threadIdx.x == 0) {
       char* r = (char*)raw;
       bulk_load(r, w0 + row0 * WS::W0, (uint32_t)(nt * WS::W0 * 2), bar);
-      if constexpr (MODE != GSB_WEIGHTS_FULL) {
-        r += nt * WS::W0 * 2;
-        bulk_load(r, wa + row0 * WS::WA, (uint32_t)(nt * WS::WA * 2), bar);
-        r += nt * WS::WA * 2;
-        bulk_load(r, wb + row0 * WS::WB, (uint32_t)(nt * WS::WB * 2), bar);
-      }
-    }
-  } else if constexpr (MODE == GSB_WEIGHTS_FULL) {
-    // one copy per row, into the odd-float4 stride
-    float* dst = (float*)S.w0;
-    if (bulk) {
-      bulk_load(dst + threadIdx.x * WS::W0S, w0 + (row0 + threadIdx.x) * WS::W0,
-                (uint32_t)(WS::W0 * sizeof(T)), bar);
-    } else {
-      const int64_t rows = min((int64_t)nt, n - row0);
-      for (int e = threadIdx.x; e < rows * WS::W0; e += nt) {
-        const int r = e / WS::W0, c = e - r * WS::W0;
-        dst[r * WS::W0S + c] = ld(w0, row0 * WS::W0 + e);
-      }
+      r += nt * WS::W0 * 2;
+      bulk_load(r, wa + row0 * WS::WA, (uint32_t)(nt * WS::WA * 2), bar);
+      r += nt * WS::WA * 2;
+      bulk_load(r, wb + row0 * WS::WB, (uint32_t)(nt * WS::WB * 2), bar);
     }
   } else {
     stage_rows<WS::W0>(w0, row0, n, (float*)S.w0, bulk, bar);
@@ -173,17 +176,6 @@ __device__ __forceinline__ void bf16_rows_to_float(const __nv_bfloat16* src, flo
   for (int e = threadIdx.x; e < count; e += blockDim.x) dst[e] = __bfloat162float(src[e]);
 }
 
-// Palette weights of one Gaussian from its staged parameter rows.
-template <int MODE, int K, int P, int Q, int R>
-__device__ __forceinline__ void weights_of(const float* w0, const float* wa, const float* wb,
-                                           const float* Y, float* w) {
-  if constexpr (MODE == GSB_WEIGHTS_FULL) {
-    sh_weights_full<K>([&](int idx) { return w0[idx]; }, 16, Y, w);
-  } else {
-    lowrank_weights<K, P, Q, R>(w0, wa, wb, Y, w);
-  }
-}
-
 // ------------------------------------------------------------- forward
 // COL: the record carries the Gaussian's palette colour sum_k w_k pal[k]
 // (3 channels) instead of its K weights -- the palette-edit render, which
@@ -203,7 +195,8 @@ __global__ void __launch_bounds__(kFuseThreads)
   pdl_wait();
   using WS = WRows<MODE, K, P, Q, R>;
   constexpr int V = RecordLayout<COL ? 3 : K>::kVec4;
-  static_assert(WS::INS >= 4 * V, "the record span reuses the input staging area");
+  using FP = FwdPlan<MODE, K, P, Q, R, T>;
+  static_assert(FP::kStaged >= 4 * V, "the record span reuses the input staging area");
   extern __shared__ __align__(16) float sm[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t warp_tot[kFuseThreads / 32], warp_max[kFuseThreads / 32];
@@ -214,32 +207,11 @@ __global__ void __launch_bounds__(kFuseThreads)
   }
   const int nt = blockDim.x, t = threadIdx.x;
   const int64_t row0 = (int64_t)blockIdx.x * nt;
-  float* raw = sm + nt * WS::INS;
+  float* raw = sm + nt * FP::kStaged;
   const int how = stage_params<MODE, K, P, Q, R, T>(n, row0, pws, rots, scales, alphas, w0, wa,
                                                     wb, sm, raw, &bar);
   const bool staged = how != kStageFailed;
-  const Staged<MODE, K, P, Q, R> S(sm);
-  if constexpr (sizeof(T) == 2) {  // raw BF16 colour rows -> their float rows
-    if (how == kStagedRawBf16) {
-      const __nv_bfloat16* r = (const __nv_bfloat16*)raw;
-      if constexpr (MODE == GSB_WEIGHTS_FULL) {
-        // 8 values (16 bytes) at a time into the odd-float4 stride
-        constexpr int C8 = WS::W0 / 8;
-        for (int e = t; e < nt * C8; e += nt) {
-          const int rr = e / C8, c = e - rr * C8;
-          const uint4 v = reinterpret_cast<const uint4*>(r)[e];
-          const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-          const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
-          const float2 c2 = __bfloat1622float2(h[2]), d = __bfloat1622float2(h[3]);
-          float4* dst = reinterpret_cast<float4*>((float*)S.w0 + rr * WS::W0S + 8 * c);
-          dst[0] = make_float4(a.x, a.y, b.x, b.y);
-          dst[1] = make_float4(c2.x, c2.y, d.x, d.y);
-        }
-      }
-      // (low-rank BF16 factors are read raw: their row strides are odd)
-    }
-    if constexpr (MODE == GSB_WEIGHTS_FULL) __syncthreads();
-  }
+  const Staged<MODE, K, P, Q, R, T> S(sm);
   const int64_t i = row0 + t;
   uint32_t cnt = 0, dk = 0;
   float f[4 * V];  // this Gaussian's record (kept until the block writes its records)
@@ -268,16 +240,26 @@ __global__ void __launch_bounds__(kFuseThreads)
           view_direction(pw, make_float3(cr.c[0], cr.c[1], cr.c[2]), dir, nullptr, nullptr);
           sh_basis(dir, WS::L + 1, Y);
           if constexpr (MODE == GSB_WEIGHTS_FULL) {
-            // the row as float4s (conflict-free at the odd-float4 stride)
+            // the row 16 bytes at a time (conflict-free at the odd stride)
             float row[WS::W0];
-            const float4* src = reinterpret_cast<const float4*>(S.w0 + t * WS::W0S);
+            const uint4* src = reinterpret_cast<const uint4*>(S.w0 + t * FP::kW0);
 #pragma unroll
-            for (int c = 0; c < WS::W0 / 4; ++c) {
-              const float4 v = src[c];
-              row[4 * c] = v.x;
-              row[4 * c + 1] = v.y;
-              row[4 * c + 2] = v.z;
-              row[4 * c + 3] = v.w;
+            for (int u = 0; u < FP::kRowUnits; ++u) {
+              const uint4 v = src[u];
+              if constexpr (sizeof(T) == 2) {
+                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const float2 x = __bfloat1622float2(h[e]);
+                  row[8 * u + 2 * e] = x.x;
+                  row[8 * u + 2 * e + 1] = x.y;
+                }
+              } else {
+                row[4 * u] = __uint_as_float(v.x);
+                row[4 * u + 1] = __uint_as_float(v.y);
+                row[4 * u + 2] = __uint_as_float(v.z);
+                row[4 * u + 3] = __uint_as_float(v.w);
+              }
             }
             sh_weights_full<K>([&](int idx) { return row[idx]; }, 16, Y, w);
           } else if (sizeof(T) == 2 && how == kStagedRawBf16) {
@@ -285,8 +267,8 @@ __global__ void __launch_bounds__(kFuseThreads)
             lowrank_weights<K, P, Q, R>(r + t * WS::W0, r + nt * WS::W0 + t * WS::WA,
                                         r + nt * (WS::W0 + WS::WA) + t * WS::WB, Y, w);
           } else {
-            weights_of<MODE, K, P, Q, R>(S.w0 + t * WS::W0, S.wa + t * WS::WA, S.wb + t * WS::WB,
-                                         Y, w);
+            lowrank_weights<K, P, Q, R>(S.w0 + t * WS::W0, S.wa + t * WS::WA, S.wb + t * WS::WB, Y,
+                                        w);
           }
           record_head(p.ux, p.uy, conic[0], conic[1], conic[2], S.al[t], f);
           if constexpr (COL) {
@@ -833,7 +815,7 @@ static int set_smem(Kern kern, int smem) {
 template <int MODE, int K, int P, int Q, int R, typename T>
 static int launch_fused(const FusedArgs& f, bool backward, cudaStream_t st) {
   using WS = WRows<MODE, K, P, Q, R>;
-  const int smem = (WS::INS + FwdExtra<MODE, K, P, Q, R, T>::kRawFloats) * kFuseThreads * 4;
+  const int smem = FwdPlan<MODE, K, P, Q, R, T>::kFloats * kFuseThreads * 4;
   const int grid = div_up(f.n, kFuseThreads);
   int rc;
   if (!backward) {
