@@ -167,6 +167,12 @@ __global__ void __launch_bounds__(kBinBlock)
 // preprocess) each block's count is first summed from its kBinBlock /
 // kPartBlock parts, and stats[1] (largest depth key) and the other stats
 // words are written here too, so that nothing needs zeroing beforehand.
+// One block; its time is load latency, so the parts are read four to a load and
+// several loads at a time: 3M Gaussians 0.023 -> 0.013 ms, 1M 0.010 -> 0.006.
+__device__ __forceinline__ uint4 load4_below(const uint32_t* p, int64_t j, int64_t n) {
+  if (j + 3 < n) return *reinterpret_cast<const uint4*>(p + j);  // p 16-byte aligned, j % 4 == 0
+  return make_uint4(j < n ? p[j] : 0u, j + 1 < n ? p[j + 1] : 0u, j + 2 < n ? p[j + 2] : 0u, 0u);
+}
 __global__ void __launch_bounds__(1024) k_scan_block_sums(uint32_t* __restrict__ sums, int64_t nb,
                                                           uint32_t* __restrict__ stats,
                                                           const uint32_t* __restrict__ psum,
@@ -174,13 +180,21 @@ __global__ void __launch_bounds__(1024) k_scan_block_sums(uint32_t* __restrict__
                                                           int64_t nparts) {
   pdl_wait();
   constexpr int kPer = kBinBlock / kPartBlock;
+  static_assert(kPer == 4, "a block's parts are one load");
   __shared__ uint32_t warp_tot[32];
   __shared__ unsigned long long carry;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (threadIdx.x == 0) carry = 0ull;
   if (psum) {
     uint32_t m = 0;
-    for (int64_t j = threadIdx.x; j < nparts; j += 1024) m = max(m, pmax[j]);
+    constexpr int kAhead = 4;
+    for (int64_t j = 4 * threadIdx.x; j < nparts; j += 4096 * kAhead) {
+      uint4 v[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) v[u] = load4_below(pmax, j + 4096 * u, nparts);
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) m = max(max(m, max(v[u].x, v[u].y)), max(v[u].z, v[u].w));
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     if (lane == 0) warp_tot[w] = m;
@@ -199,13 +213,8 @@ __global__ void __launch_bounds__(1024) k_scan_block_sums(uint32_t* __restrict__
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       if (psum) {
-        uint32_t t = 0;
-#pragma unroll
-        for (int q = 0; q < kPer; ++q) {
-          const int64_t pj = (j0 + k) * kPer + q;
-          t += pj < nparts ? psum[pj] : 0u;
-        }
-        v[k] = (j0 + k < nb) ? t : 0u;
+        const uint4 q = load4_below(psum, (j0 + k) * kPer, nparts);
+        v[k] = (j0 + k < nb) ? q.x + q.y + q.z + q.w : 0u;
       } else {
         v[k] = (j0 + k < nb) ? sums[j0 + k] : 0u;
       }
