@@ -90,13 +90,12 @@ struct SsimScales {
   float w_l1;      // (1 - lambda_ssim) / (3 H W)
   float w_ssim;    // lambda_ssim / (3 H W)
   float w_pos;     // lambda_pos / (K H W)
+  float lambda_ssim;
 };
 
-__global__ void k_l1_ssim_init(float* __restrict__ loss, float* __restrict__ dpal, int n_pal,
-                               float lambda_ssim) {
+__global__ void k_l1_ssim_init(float* __restrict__ loss, float* __restrict__ dpal, int n_pal) {
   pdl_wait();
-  // total = lambda_ssim * (1 - mean SSIM) + ...: the blocks add -w_ssim * sum S
-  if (threadIdx.x < 4) loss[threadIdx.x] = threadIdx.x == 0 ? lambda_ssim : 0.f;
+  if (threadIdx.x < 4) loss[threadIdx.x] = 0.f;
   if (dpal && threadIdx.x < n_pal) dpal[threadIdx.x] = 0.f;
 }
 
@@ -423,18 +422,22 @@ __global__ void __launch_bounds__(kSsimThreads, kSsimBlocks)
     float v = 0.f;
 #pragma unroll
     for (int k = 0; k < kSsimRole / 32; ++k) v += red[(tid == 1 ? 0 : kSsimRole / 32) + k][tid];
-    if (tid == 0) {
-      atomicAdd(loss + 1, v * sc.inv_n);
-      atomicAdd(loss, v * sc.w_l1);
-    } else if (tid == 1) {
-      atomicAdd(loss + 2, v * sc.inv_n);
-      atomicAdd(loss, -v * sc.w_ssim);
-    } else if (tid == 2) {
-      atomicAdd(loss + 3, v * sc.w_pos);
-      atomicAdd(loss, v * sc.w_pos);
-    } else if (dpal) {
+    if (tid < 3)
+      atomicAdd(loss + 1 + tid, v * (tid == 2 ? sc.w_pos : sc.inv_n));
+    else if (dpal)
       atomicAdd(dpal + (tid - 3), v);
-    }
+    __threadfence();
+  }
+  __syncthreads();
+  // The block that finishes last forms the total from the three sums: a total
+  // added up block by block would round three times as often, at a larger value.
+  // Until then loss[0] counts the blocks.
+  if (tid == 0 && atomicAdd(reinterpret_cast<unsigned*>(loss), 1u) ==
+                      gridDim.x * gridDim.y - 1) {
+    __threadfence();
+    const volatile float* part = loss;
+    loss[0] = (float)((double)sc.lambda_ssim * (1.0 - (double)part[2]) +
+                      (1.0 - (double)sc.lambda_ssim) * (double)part[1] + (double)part[3]);
   }
 }
 
@@ -481,10 +484,10 @@ int launch_palette_l1_ssim(int K, int H, int W, const float* layer, const float*
   sc.inv_n = hw ? (float)(1.0 / (3.0 * (double)hw)) : 0.f;
   sc.w_l1 = (1.f - lambda_ssim) * sc.inv_n;
   sc.w_ssim = lambda_ssim * sc.inv_n;
+  sc.lambda_ssim = lambda_ssim;
   sc.w_pos = hw ? (float)((double)lambda_pos / ((double)K * (double)hw)) : 0.f;
   // an empty image has no pixels to average: its loss and gradients are 0
-  launch_pdl(k_l1_ssim_init, dim3(1), dim3(32), 0, st, loss, dpal, 3 * K,
-             hw ? lambda_ssim : 0.f);
+  launch_pdl(k_l1_ssim_init, dim3(1), dim3(32), 0, st, loss, dpal, 3 * K);
   int rc = check_launch("palette_l1_ssim (init)");
   if (rc || hw == 0) return rc;
   // Segments of 11 s - 20 rows take s steps and one to finish; the blocks that
