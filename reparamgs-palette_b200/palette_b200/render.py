@@ -198,11 +198,30 @@ def _weight_args(shs, dc, A, B, K):
     if not (dc.dtype == A.dtype == B.dtype):
         raise TypeError("render_palette: dc, A and B must share a dtype")
     K = int(dc.shape[1])
-    if A.dim() == 2:
+    if A.dim() == 2 and B.dim() == 2:
         P, rank, Q = int(A.shape[1]), 1, int(B.shape[1])
-    else:
+    elif A.dim() == 3 and B.dim() == 3:
         P, rank, Q = int(A.shape[1]), int(A.shape[2]), int(B.shape[2])
+        if int(B.shape[1]) != rank:
+            raise ValueError(f"render_palette: B must be [N, {rank}, Q], got {tuple(B.shape)}")
+    else:
+        raise ValueError("render_palette: A and B must both be 2-D (rank 1) or 3-D (rank r)")
     return dc, A, B, _lib.WEIGHTS_LOWRANK, K, P, Q, rank
+
+
+def _check_rows(pws, rots, scales, alphas, w0, A, B, mode, K, P, Q, rank):
+    """The kernels read (and the adjoint writes) pws.shape[0] rows of every
+    parameter: refuse a tensor that holds fewer elements."""
+    n = int(pws.shape[0])
+    rows = [("pws", pws, 3), ("rots", rots, 4), ("scales", scales, 3), ("alphas", alphas, 1)]
+    if mode == _lib.WEIGHTS_FULL:
+        rows.append(("shs", w0, 16 * K))
+    else:
+        rows += [("dc", w0, K), ("A", A, P * rank), ("B", B, rank * Q)]
+    for name, t, width in rows:
+        if t.numel() < n * width:
+            raise ValueError(f"render_palette: {name} {tuple(t.shape)} has fewer than {n} rows of "
+                             f"{width}")
 
 
 def render_palette(pws, rots, scales, alphas, cam, shs=None, dc=None, A=None, B=None, K=None):
@@ -212,6 +231,7 @@ def render_palette(pws, rots, scales, alphas, cam, shs=None, dc=None, A=None, B=
     pws, rots, scales = _check("pws", pws), _check("rots", rots), _check("scales", scales)
     alphas = _check("alphas", alphas)
     w0, A, B, mode, K, P, Q, rank = _weight_args(shs, dc, A, B, K)
+    _check_rows(pws, rots, scales, alphas, w0, A, B, mode, K, P, Q, rank)
     if not (torch.is_grad_enabled() and any(
             t is not None and t.requires_grad for t in (pws, rots, scales, alphas, w0, A, B))):
         # nothing to differentiate: render without the autograd node
@@ -298,6 +318,7 @@ def render_palette_views(pws, rots, scales, alphas, cams, shs=None, dc=None, A=N
     if not cams:
         raise ValueError("render_palette_views: no cameras")
     w0, A, B, mode, K, P, Q, rank = _weight_args(shs, dc, A, B, K)
+    _check_rows(pws, rots, scales, alphas, w0, A, B, mode, K, P, Q, rank)
     out = _RenderPaletteViews.apply(pws, rots, scales, alphas, w0, A, B, cams, mode, K, P, Q, rank)
     V = len(cams)
     return list(out[:V]), list(out[V:2 * V]), list(out[2 * V:])

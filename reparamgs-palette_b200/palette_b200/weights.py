@@ -34,7 +34,7 @@ import torch
 import gsplatcu as gsc
 from gsplatcu import _lib
 
-from .render import _params, _render_one, _weight_args, camera_struct
+from .render import _check_rows, _params, _render_one, _weight_args, camera_struct
 
 _F32 = torch.float32
 
@@ -118,5 +118,6 @@ def splat_palette_weights(pws, alphas, scales, rots, cam, shs=None, dc=None, A=N
     for name in ("Rcw", "tcw", "twc"):
         gsc._cuda("splat_palette_weights", name, getattr(cam, name))
     w0, A, B, mode, K, P, Q, rank = _weight_args(shs, dc, A, B, K)
+    _check_rows(pws, rots, scales, alphas, w0, A, B, mode, K, P, Q, rank)
     return _SplatWeights.apply(pws.contiguous(), alphas.contiguous(), scales.contiguous(),
                                rots.contiguous(), w0, A, B, cam, mode, K, P, Q, rank)
