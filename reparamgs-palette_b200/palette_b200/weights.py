@@ -58,11 +58,20 @@ def _operator_chain(pws, alphas, scales, rots, w0, A, B, cam, mode, K, Q):
     return layer, depths
 
 
+def _saved(t, dtype):
+    """A tensor kept from the forward, as the library reads it: saved-tensor hooks
+    may have handed back another layout (made dense) or type (refused)."""
+    if t.dtype != dtype or not t.is_cuda:
+        raise TypeError(f"splat_palette_weights: a saved tensor came back as {t.dtype} on "
+                        f"{t.device}, saved as {dtype} on a CUDA device")
+    return t.contiguous()
+
+
 class _SplatWeights(torch.autograd.Function):
     @staticmethod
     def forward(ctx, pws, alphas, scales, rots, w0, A, B, cam, mode, K, P, Q, rank):
         fused = 3 <= K <= 8 if mode == _lib.WEIGHTS_FULL else (K, P, Q, rank) in _FUSED_LOWRANK
-        ctx.meta = (cam, mode, K, P, Q, rank)
+        ctx.meta = (cam, mode, K, P, Q, rank, w0.dtype)
         if fused:
             layer, tau, depths, state, ranges, gsid, contrib = _render_one(
                 pws, rots, scales, alphas, w0, A, B, cam, mode, K, P, Q, rank)
@@ -76,13 +85,19 @@ class _SplatWeights(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dlayer, _dvisible):
-        cam, mode, K, P, Q, rank = ctx.meta
+        cam, mode, K, P, Q, rank, wt = ctx.meta
         pws, w0, A, B, state, ranges, gsid, contrib, tau = ctx.saved_tensors
         if state is None:
             raise _lib.GsplatError(
                 f"splat_palette_weights: unsupported palette parameter shape (K={K}, P={P}, Q={Q}, "
                 f"rank={rank}) in the backward (status {_lib.GSB_ERR_UNSUPPORTED})",
                 _lib.GSB_ERR_UNSUPPORTED)
+        pws, tau = _saved(pws, _F32), _saved(tau, _F32)
+        state = _saved(state, torch.uint8)
+        if state.data_ptr() % 256:
+            state = state.clone()
+        ranges, gsid, contrib = (_saved(t, torch.int32) for t in (ranges, gsid, contrib))
+        w0, A, B = (None if t is None else _saved(t, wt) for t in (w0, A, B))
         dev = pws.device
         n = int(pws.shape[0])
         camst, _keep = camera_struct(cam)
