@@ -2,6 +2,7 @@
 // argument validation, workspace carving and kernel launches.  No entry point
 // allocates device memory or synchronises, except gsb_splat_counts, which
 // must return the patch count to the host.
+#include <algorithm>
 #include <mutex>
 #include <cmath>
 #include <atomic>
@@ -303,25 +304,35 @@ GSB_API int gsb_splat_counts(int64_t n, int height, int width, const void* state
   return GSB_OK;
 }
 
-// The depth-ordered fill passes over every patch once, the radix sort 3 or 4 times,
-// but it has more launches and a pass over every Gaussian: 0.128 against 0.169 ms
-// at 3.3M patches (1M Gaussians, 1080p), 0.56 against 1.11 ms at 20.8M (3M, 4K),
-// 0.080 against 0.087 ms at 1.3M, 0.033 against 0.029 ms at 0.6M (250k, 720p),
-// 0.047 against 0.041 ms at 30k.
-constexpr int64_t kTileListPatches = 1500000;
-static bool use_tile_lists(const ListPlan& p) { return p.ok && p.M >= kTileListPatches; }
-
-// Workspace of either path (the choice between them is not the caller's).
-static size_t tile_sort_bytes(int64_t n, int height, int width, int64_t patches,
-                              uint32_t max_depth_key) {
-  const size_t radix = make_sort_plan(n, height, width, patches, max_depth_key).bytes_total;
-  const ListPlan p = make_list_plan(n, height, width, patches, max_depth_key);
-  return use_tile_lists(p) && p.bytes_total > radix ? p.bytes_total : radix;
+// Depth-ordered lists or radix sort over patches?  The lists write every patch
+// once, where the radix sort makes 3 to 5 passes over all of them; but they also
+// pass over the Gaussians, once per band of tile rows, and every band of every
+// chunk costs its counters.  Both times in microseconds, for N million Gaussians,
+// M million patches and b bands, fitted within 10 % to 270 measured sizes (0.1 to
+// 10M Gaussians, 0.6 to 90M patches, 256x256 to 8K, 12000x2000, 2000x8000); rows
+// wider than 480 tiles (8K) lengthen a band's serial row sums.  Radix / lists:
+//   1080p, 3 bands:  1M, 4.3M patches 196 / 117;  3M, 6.0M 279 / 219;  1M, 1.3M 81 / 103
+//   4K,   12 bands:  3M, 27.5M 1327 / 489;  1M, 4.3M 226 / 198;  1M, 2.0M 130 / 188
+//   8K,   68 bands:  3M, 90M 4347 / 2045;  3M, 27.9M 1357 / 1264;  3M, 6.1M 328 / 1162
+// Over those sizes the rule costs at most 7 % against the faster path.  Below 1.2M
+// patches neither gains 15 us and the radix sort stays (0.6M, 250k Gaussians,
+// 720p: 29 against 33 us; 30k patches: 41 against 47).  The workspace is the radix
+// sort's, as callers size it: lists that need more (few patches per Gaussian, or
+// counters of many tiles) are not taken.  `patches`: of a capacity, the four fifths
+// that the package's own capacities (1.25 times the count seen) hold.
+static bool use_tile_lists(const ListPlan& l, const SortPlan& r, double patches) {
+  if (!l.ok || l.bytes_total > r.bytes_total || patches < 1.2e6) return false;
+  const double N = (double)l.n * 1e-6, M = patches * 1e-6;
+  const double b = l.bands * std::max(1.0, l.gx / 480.0);
+  const double beyond_l2 = 20.0 * std::max(0.0, N - 5.0);  // sort buffers of > 120 MB
+  const double lists = 34.0 + 5.0 * b + N * (10.0 + 3.3 * b + 12.0 * l.passes) + beyond_l2 + 5.0 * M;
+  const double radix = 28.0 + 2.0 * r.passes + 12.0 * r.passes * M;
+  return 1.03 * lists < radix;
 }
 
 GSB_API size_t gsb_splat_sort_bytes(int64_t n, int height, int width, const gsb_splat_plan* plan) {
   if (n < 0 || height < 0 || width < 0 || !plan || plan->patches < 0) return 0;
-  return tile_sort_bytes(n, height, width, plan->patches, plan->max_depth_key);
+  return make_sort_plan(n, height, width, plan->patches, plan->max_depth_key).bytes_total;
 }
 
 GSB_API int gsb_splat_sort(int64_t n, int height, int width, const gsb_splat_plan* plan,
@@ -336,7 +347,7 @@ GSB_API int gsb_splat_sort(int64_t n, int height, int width, const gsb_splat_pla
   const SortPlan p = make_sort_plan(n, height, width, plan->patches, plan->max_depth_key);
   const SplatState s = carve_state((void*)state, n, 1, height, width);
   const ListPlan lp = make_list_plan(n, height, width, plan->patches, plan->max_depth_key);
-  if (use_tile_lists(lp))
+  if (use_tile_lists(lp, p, (double)plan->patches))
     return launch_tile_lists(lp, s, sort_ws, gsid_out, ranges_out, nullptr, ST(stream));
   return launch_sort(p, n, height, width, s, sort_ws, gsid_out, ranges_out, ST(stream));
 }
@@ -344,7 +355,7 @@ GSB_API int gsb_splat_sort(int64_t n, int height, int width, const gsb_splat_pla
 GSB_API size_t gsb_splat_sort_capacity_bytes(int64_t n, int height, int width,
                                              int64_t patch_capacity, uint32_t max_depth_key) {
   if (n < 0 || height < 0 || width < 0 || patch_capacity < 0) return 0;
-  return tile_sort_bytes(n, height, width, patch_capacity, max_depth_key);
+  return make_sort_plan(n, height, width, patch_capacity, max_depth_key).bytes_total;
 }
 
 GSB_API int gsb_splat_patch_status(int64_t n, int height, int width, int64_t patch_capacity,
@@ -372,7 +383,7 @@ GSB_API int gsb_splat_sort_capacity(int64_t n, int height, int width, int64_t pa
   const SortPlan p = make_sort_plan(n, height, width, patch_capacity, max_depth_key);
   const SplatState s = carve_state((void*)state, n, 1, height, width);
   const ListPlan lp = make_list_plan(n, height, width, patch_capacity, max_depth_key);
-  if (use_tile_lists(lp)) {
+  if (use_tile_lists(lp, p, 0.8 * (double)patch_capacity)) {
     if (status && (rc = launch_patch_status(p, s, status, ST(stream)))) return rc;
     return launch_tile_lists(lp, s, sort_ws, gsid_out, ranges_out, s.stats, ST(stream));
   }
