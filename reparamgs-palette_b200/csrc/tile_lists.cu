@@ -41,6 +41,15 @@ constexpr int kMaxChunks = 148;     // one block per SM and band
 
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
+// Dynamic shared memory limits of the kernels: the same for every image, since the
+// attribute belongs to the function and host threads render different sizes at the
+// same time.  A band of the fill has at most kBandCells cells and rows of at most
+// kMaxPitch.
+constexpr int kMaxPitch = kBandCells / kRowGroup;
+constexpr int kCountSmemMax = kCountCells * 4;
+constexpr int kFillSmemMax = (kBandCells + kListWarps * (kBandCells + kMaxPitch) / 2) * 4;
+constexpr int kSortSmem = kSortTile * 8 + (8 * kRadixBins + 2 * kRadixBins + 8) * 4;
+
 static int bits_of(uint32_t v) { return v ? 32 - __builtin_clz(v) : 0; }
 
 // Tile rows are dealt to the bands in groups of kRowGroup, so that the bands of
@@ -61,6 +70,12 @@ struct BandRows {
     return q * kRowGroup + (in < 0 ? 0 : in > kRowGroup ? kRowGroup : in);
   }
 };
+
+// Dynamic shared memory of an image's counting and filling blocks.
+static size_t count_bytes(const ListPlan& p) { return (size_t)(p.count_rows + 1) * (p.gx + 1) * 4; }
+static size_t fill_bytes(const ListPlan& p) {
+  return (size_t)(p.band_rows * p.pitch + kListWarps * ((p.band_rows + 1) * p.pitch / 2)) * 4;
+}
 
 ListPlan make_list_plan(int64_t n, int H, int W, int64_t M, uint32_t max_dkey) {
   ListPlan p{};
@@ -90,6 +105,7 @@ ListPlan make_list_plan(int64_t n, int H, int W, int64_t M, uint32_t max_dkey) {
          (BandRows(0, p.count_bands).below(p.gy) + 1) * (p.gx + 1) > kCountCells)
     ++p.count_bands;
   p.count_rows = BandRows(0, p.count_bands).below(p.gy);
+  p.ok = count_bytes(p) <= kCountSmemMax && fill_bytes(p) <= kFillSmemMax;  // (every image's)
   p.sort_blocks = (n + kSortTile - 1) / kSortTile;
   p.groups = (n + kGroupSize - 1) / kGroupSize;
   size_t off = 0;
@@ -549,21 +565,15 @@ int launch_tile_lists(const ListPlan& p, const SplatState& s, void* ws, int32_t*
   uint32_t* counts = (uint32_t*)(b + p.off_counts);
   uint32_t* tile_tot = (uint32_t*)(b + p.off_tile_tot);
   const int nbk = (int)p.sort_blocks;
-  const size_t sort_smem =
-      (size_t)kSortTile * 8 + (8 * kRadixBins + 2 * kRadixBins + 8) * 4;
-  const int starts = p.band_rows * p.pitch, words = (p.band_rows + 1) * p.pitch / 2;
-  const size_t count_smem = (size_t)(p.count_rows + 1) * (p.gx + 1) * 4;
-  const size_t list_smem = (size_t)(starts + kListWarps * words) * 4;
-  if (cudaFuncSetAttribute(k_radix_downsweep<uint32_t, kVisible>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sort_smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_radix_downsweep<uint32_t, kDevice>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sort_smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_tile_counts, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)count_smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_tile_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)list_smem) != cudaSuccess)
+  const size_t count_smem = count_bytes(p), list_smem = fill_bytes(p);
+  const auto limit = [](const void* kern, int bytes) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) ==
+           cudaSuccess;
+  };
+  if (!limit((const void*)k_radix_downsweep<uint32_t, kVisible>, kSortSmem) ||
+      !limit((const void*)k_radix_downsweep<uint32_t, kDevice>, kSortSmem) ||
+      !limit((const void*)k_tile_counts, kCountSmemMax) ||
+      !limit((const void*)k_tile_scatter, kFillSmemMax))
     return check_launch("tile lists (shared memory attribute)", 0);
   // 1. depth order of the Gaussians that have patches
   int src = 0;
@@ -576,7 +586,7 @@ int launch_tile_lists(const ListPlan& p, const SplatState& s, void* ws, int32_t*
                  (const uint32_t*)s.dkeys, p.n, shift, mask, hist, p.sort_blocks,
                  (const uint32_t*)nullptr, (const uint32_t*)s.counts);
       launch_pdl(k_radix_scan, dim3(mask + 1), dim3(256), 0, st, hist, p.sort_blocks, dtot);
-      launch_pdl(k_radix_downsweep<uint32_t, kVisible>, dim3(nbk), dim3(kSortThreads), sort_smem,
+      launch_pdl(k_radix_downsweep<uint32_t, kVisible>, dim3(nbk), dim3(kSortThreads), kSortSmem,
                  st, (const uint32_t*)s.dkeys, (const int32_t*)nullptr, keys[0], vals[0], p.n, shift,
                  mask, (const uint32_t*)hist, (const uint32_t*)dtot, p.sort_blocks,
                  (const uint32_t*)nullptr, (const uint32_t*)s.counts, visible);
@@ -585,7 +595,7 @@ int launch_tile_lists(const ListPlan& p, const SplatState& s, void* ws, int32_t*
                  (const uint32_t*)keys[src], p.n, shift, mask, hist, p.sort_blocks,
                  (const uint32_t*)visible, (const uint32_t*)nullptr);
       launch_pdl(k_radix_scan, dim3(mask + 1), dim3(256), 0, st, hist, p.sort_blocks, dtot);
-      launch_pdl(k_radix_downsweep<uint32_t, kDevice>, dim3(nbk), dim3(kSortThreads), sort_smem, st,
+      launch_pdl(k_radix_downsweep<uint32_t, kDevice>, dim3(nbk), dim3(kSortThreads), kSortSmem, st,
                  (const uint32_t*)keys[src], (const int32_t*)vals[src], keys[src ^ 1],
                  vals[src ^ 1], p.n, shift, mask, (const uint32_t*)hist, (const uint32_t*)dtot,
                  p.sort_blocks, (const uint32_t*)visible, (const uint32_t*)nullptr,
