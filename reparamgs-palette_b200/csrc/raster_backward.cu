@@ -308,6 +308,35 @@ __device__ __forceinline__ void adjoint_geom_pair(BwdPixel<K> (&p)[NP], int base
   }
 }
 
+// Stages the records [base, base + cnt) of a tile's list, with their block masks.
+template <int K, bool GEOM, int NP>
+__device__ __forceinline__ void stage_batch(const int32_t* __restrict__ gsid,
+                                            const float4* __restrict__ records, int first, int cnt,
+                                            int X0, int Y0, float4* srec, int32_t* sgid,
+                                            uint8_t* smask) {
+  using L = AdjLayout<NP>;
+  constexpr int V = RecordLayout<K>::kVec4;
+  for (int t = threadIdx.x; t < cnt; t += L::kThreads) {
+    const int g = gsid[first + t];
+    const float4* src = records + (int64_t)g * V;
+    const float4 v0 = __ldg(src), v1 = __ldg(src + 1), v2 = __ldg(src + 2);
+    srec[t] = v0;
+    srec[kBatch + t] = v1;
+#pragma unroll
+    for (int v = 3; v < V; ++v)
+      if (GEOM) srec[(v - 1) * kBatch + t] = __ldg(src + v);
+    sgid[t] = g;
+    smask[t] = (uint8_t)region_mask<2, L::kBands, 8, L::kRows>(v0, v1, v2, X0, Y0);
+  }
+}
+
+// Incoming gradients above this (infinite ones and NaN among them) leave the scalar
+// recursion: dl . f would overflow, and inf - inf is NaN where the blended features
+// of each channel stay finite and give signed infinities.  (A feature that is itself
+// infinite gives its pixels' contributors infinite or NaN gradients either way.)
+constexpr float kTame = 1e30f;
+constexpr int kWild = 0x7fffffff;  // as a tile's largest contributor index
+
 // Walks each pixel's contributors back to front from its `contrib` index,
 // recovering T by division by (1 - alpha') from the saved final T.  The
 // per-pixel skip decisions use the forward's exact expressions, so the walk
@@ -328,7 +357,7 @@ __global__ void __launch_bounds__(AdjLayout<NP>::kThreads,
                                   (GEOM ? (K == 4 || K == 5 ? 7 : 6) : 8) * NP / 2)
     k_draw_backward(int H, int W, int gx, const int2* __restrict__ ranges,
                     const int32_t* __restrict__ gsid, const float4* __restrict__ records,
-                    const int32_t* __restrict__ order,
+                    int32_t* __restrict__ order,
                     const int32_t* __restrict__ contrib, const float* __restrict__ final_tau,
                     const float* __restrict__ dout, const float* __restrict__ dtau,
                     float* __restrict__ dfeat, float* __restrict__ dalpha,
@@ -343,6 +372,7 @@ __global__ void __launch_bounds__(AdjLayout<NP>::kThreads,
   __shared__ uint8_t smask[kBatch];
   __shared__ unsigned s_maxc;
   const int tile = order[blockIdx.x];
+  if (tile < 0) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int X0 = (tile % gx) * kTile, Y0 = (tile / gx) * kTile;
   const int px = X0 + (w & 1) * 8 + (lane & 7);
@@ -353,6 +383,7 @@ __global__ void __launch_bounds__(AdjLayout<NP>::kThreads,
   BwdPixel<K> p[NP];
   float fy[NP];
   int wmax = 0;
+  bool tame = true;
 #pragma unroll
   for (int q = 0; q < NP; ++q) {
     const bool in = px < W && py + 4 * q < H;
@@ -364,12 +395,22 @@ __global__ void __launch_bounds__(AdjLayout<NP>::kThreads,
     p[q].R = (GEOM && dtau && in) ? dtau[pix] : 0.f;
     p[q].cont = in ? contrib[pix] : 0;
     wmax = max(wmax, p[q].cont);
+    if constexpr (GEOM) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) tame &= fabsf(p[q].dl[k]) <= kTame;
+      tame &= fabsf(p[q].R) <= kTame;
+    }
   }
+  if (GEOM && !tame) wmax = kWild;
   wmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)wmax);
   if (threadIdx.x == 0) s_maxc = 0u;
   __syncthreads();
   if (lane == 0) atomicMax(&s_maxc, (unsigned)wmax);
   __syncthreads();
+  if (GEOM && (int)s_maxc == kWild) {  // k_draw_backward_wild's
+    if (threadIdx.x == 0) order[blockIdx.x] = ~tile;
+    return;
+  }
   // contributor indices never exceed the tile's list (clamped for safety
   // against mismatched inputs)
   const int maxc = min((int)s_maxc, rg.y - rg.x);
@@ -378,18 +419,7 @@ __global__ void __launch_bounds__(AdjLayout<NP>::kThreads,
     const int base = max(0, top - kBatch);
     const int cnt = top - base;
     __syncthreads();
-    for (int t = threadIdx.x; t < cnt; t += L::kThreads) {
-      const int g = gsid[rg.x + base + t];
-      const float4* src = records + (int64_t)g * V;
-      const float4 v0 = __ldg(src), v1 = __ldg(src + 1), v2 = __ldg(src + 2);
-      srec[t] = v0;
-      srec[kBatch + t] = v1;
-#pragma unroll
-      for (int v = 3; v < V; ++v)
-        if (GEOM) srec[(v - 1) * kBatch + t] = __ldg(src + v);
-      sgid[t] = g;
-      smask[t] = (uint8_t)region_mask<2, L::kBands, 8, L::kRows>(v0, v1, v2, X0, Y0);
-    }
+    stage_batch<K, GEOM, NP>(gsid, records, rg.x + base, cnt, X0, Y0, srec, sgid, smask);
     __syncthreads();
     const int hi = min(cnt, wmax - base);
     for (int s_hi = hi; s_hi > 0; s_hi -= 32) {
@@ -449,6 +479,92 @@ __global__ void __launch_bounds__(AdjLayout<NP>::kThreads,
   }
 }
 
+// Full adjoint of the tiles that k_draw_backward left out (kTame; it marks them in
+// the launch order), with the features blended behind each record kept per channel:
+// the terms as the reference forms them.  One pixel per thread.  A launch of its own,
+// of kWildTiles tiles per block: as a call inside k_draw_backward it cost that kernel
+// registers and 2 to 4 % (500k, 1080p, K = 5: 526 -> 537 us; K = 3: 424 -> 443).
+constexpr int kWildTiles = 8;
+template <int K>
+__global__ void __launch_bounds__(kTilePixels)
+    k_draw_backward_wild(int tiles, int H, int W, int gx, const int2* __restrict__ ranges,
+                         const int32_t* __restrict__ gsid, const float4* __restrict__ records,
+                         const int32_t* __restrict__ order, const int32_t* __restrict__ contrib,
+                         const float* __restrict__ final_tau, const float* __restrict__ dout,
+                         const float* __restrict__ dtau, float* __restrict__ dfeat,
+                         float* __restrict__ dalpha, float* __restrict__ du,
+                         float* __restrict__ dconic) {
+  pdl_wait();
+  using L = AdjLayout<1>;
+  constexpr int NREAL = K + 6;
+  __shared__ float4 srec[(RecordLayout<K>::kVec4 - 1) * kBatch];
+  __shared__ int32_t sgid[kBatch];
+  __shared__ uint8_t smask[kBatch];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t hw = (int64_t)H * W;
+  for (int e = 0; e < kWildTiles; ++e) {  // (uniform per block)
+    const int at = blockIdx.x * kWildTiles + e;
+    if (at >= tiles || order[at] >= 0) continue;
+    const int tile = ~order[at];
+    const int X0 = (tile % gx) * kTile, Y0 = (tile / gx) * kTile;
+    const int px = X0 + (w & 1) * 8 + (lane & 7), py = Y0 + (w >> 1) * L::kRows + (lane >> 3);
+    const bool in = px < W && py < H;
+    const int64_t pix = (int64_t)py * W + px;
+    const int2 rg = ranges[tile];
+    const int n = rg.y - rg.x;
+    float dl[K], G[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      dl[k] = in ? dout[k * hw + pix] : 0.f;
+      G[k] = 0.f;
+    }
+    const float Tf = in ? final_tau[pix] : 0.f, dTf = (dtau && in) ? dtau[pix] : 0.f;
+    const int cont = in ? contrib[pix] : 0;
+    float T = Tf;
+    for (int base = (n - 1) / kBatch * kBatch; base >= 0; base -= kBatch) {
+      const int cnt = min(kBatch, n - base);
+      __syncthreads();
+      stage_batch<K, true, 1>(gsid, records, rg.x + base, cnt, X0, Y0, srec, sgid, smask);
+      __syncthreads();
+      for (int j = cnt - 1; j >= 0; --j) {
+        if (!((smask[j] >> w) & 1)) continue;  // (uniform per warp)
+        const float4 v0 = srec[j], v1 = srec[kBatch + j];
+        const float dx = v0.x - (float)px, dy = v0.y - (float)py;
+        const float m = fminf(0.f, half_form(v0.z, v0.w, v1.x, dx, dy));
+        const bool hit = base + j < cont && m >= v1.y;
+        if (!__any_sync(0xffffffffu, hit)) continue;
+        float f[K], x[NREAL];
+        load_feats<K>(srec, j, v1.w, f);
+#pragma unroll
+        for (int v = 0; v < NREAL; ++v) x[v] = 0.f;
+        if (hit) {
+          const float g = expf(m), ap = fminf(kAlphaMax, v1.z * g);
+          const float one_m = 1.f - ap, inv = rcp_approx(one_m);
+          T *= inv;
+          float dap = 0.f;
+#pragma unroll
+          for (int k = 0; k < K; ++k) {
+            x[k] = dl[k] * (ap * T);
+            dap += dl[k] * (T * (f[k] - G[k]));
+            G[k] = ap * f[k] + one_m * G[k];
+          }
+          if (dtau) dap += dTf * (-Tf * inv);
+          x[K] = dap * g;
+          x[K + 1] = dap * ((2.f * v0.z * dx + v0.w * dy) * ap);
+          x[K + 2] = dap * ((v0.w * dx + 2.f * v1.x * dy) * ap);
+          x[K + 3] = dap * (-0.5f * ap * (dx * dx));
+          x[K + 4] = dap * (-1.0f * ap * (dx * dy));
+          x[K + 5] = dap * (-0.5f * ap * (dy * dy));
+        }
+        int vidx;
+        bool owner;
+        const float tot = warp_spread_sum<NREAL, 16>(x, lane, &vidx, &owner);
+        if (owner) atomicAdd(grad_slot<K>(vidx, sgid[j], dfeat, dalpha, du, dconic), tot);
+      }
+    }
+  }
+}
+
 // Up to this many tiles (4 blocks per SM) a warp is alone on its scheduler or
 // nearly so, and the time is the longest tile's chain of records: with one
 // pixel per lane it is shorter (256 tiles, 20k Gaussians: 91 -> 63 us).  On
@@ -458,7 +574,7 @@ constexpr int kOnePixelTiles = 592;
 
 template <int K>
 static void draw_bwd_k(int tiles, int H, int W, int gx, const int2* rg, const int32_t* gsid,
-                       const float4* rec, const int32_t* order, const int32_t* contrib,
+                       const float4* rec, int32_t* order, const int32_t* contrib,
                        const float* ft, const float* dout, const float* dtau, float* dfeat,
                        float* dalpha, float* du, float* dq, cudaStream_t st) {
   const bool one = tiles <= kOnePixelTiles;
@@ -466,6 +582,10 @@ static void draw_bwd_k(int tiles, int H, int W, int gx, const int2* rg, const in
                   : (dalpha ? k_draw_backward<K, true, 2> : k_draw_backward<K, false, 2>);
   launch_pdl(kern, dim3(tiles), dim3(kTilePixels / (one ? 1 : 2)), 0, st, H, W, gx, rg, gsid, rec,
              order, contrib, ft, dout, dtau, dfeat, dalpha, du, dq);
+  if (dalpha)
+    launch_pdl(k_draw_backward_wild<K>, dim3(div_up(tiles, kWildTiles)), dim3(kTilePixels), 0, st,
+               tiles, H, W, gx, rg, gsid, rec, (const int32_t*)order, contrib, ft, dout, dtau, dfeat,
+               dalpha, du, dq);
 }
 
 int launch_draw_backward(int64_t n, int H, int W, int channels, const int32_t* ranges,
@@ -490,7 +610,7 @@ int launch_draw_backward(int64_t n, int H, int W, int channels, const int32_t* r
 #undef GSB_K
     default: return GSB_ERR_INVALID_ARGUMENT;
   }
-  return check_launch("splat_backward");
+  return check_launch("splat_backward", dalpha ? 2 : 1);
 }
 
 }  // namespace gsb
