@@ -112,14 +112,9 @@ int launch_palette_l1(int K, int H, int W, const float* layer, const float* pale
 // 26 us for two broadcast multiplies in torch.
 constexpr int kScaleThreads = 256, kScaleVec = 4;
 
-__global__ void __launch_bounds__(kScaleThreads)
-    k_scale_gradients(int64_t n0, const float* __restrict__ in0, float* __restrict__ out0,
-                      int64_t n1, const float* __restrict__ in1, float* __restrict__ out1,
-                      const float* __restrict__ factor) {
-  pdl_wait();
-  const float f = *factor;
-  const int64_t vecs =
-      ((uintptr_t)in0 % 16 == 0 && (uintptr_t)out0 % 16 == 0) ? n0 / 4 : 0;
+__device__ __forceinline__ void scale_array(int64_t n, const float* __restrict__ in,
+                                            float* __restrict__ out, float f) {
+  const int64_t vecs = ((uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0) ? n / 4 : 0;
   const int64_t first = (int64_t)blockIdx.x * kScaleThreads * kScaleVec + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * kScaleThreads * kScaleVec;
   for (int64_t i = first; i < vecs; i += stride) {
@@ -127,27 +122,36 @@ __global__ void __launch_bounds__(kScaleThreads)
 #pragma unroll
     for (int k = 0; k < kScaleVec; ++k) {
       const int64_t j = i + k * kScaleThreads;
-      if (j < vecs) v[k] = reinterpret_cast<const float4*>(in0)[j];
+      if (j < vecs) v[k] = reinterpret_cast<const float4*>(in)[j];
     }
 #pragma unroll
     for (int k = 0; k < kScaleVec; ++k) {
       const int64_t j = i + k * kScaleThreads;
       if (j < vecs)
-        reinterpret_cast<float4*>(out0)[j] =
+        reinterpret_cast<float4*>(out)[j] =
             make_float4(v[k].x * f, v[k].y * f, v[k].z * f, v[k].w * f);
     }
   }
   const int64_t t = (int64_t)blockIdx.x * kScaleThreads + threadIdx.x;
   const int64_t threads = (int64_t)gridDim.x * kScaleThreads;
-  for (int64_t i = 4 * vecs + t; i < n0; i += threads) out0[i] = in0[i] * f;
-  for (int64_t i = t; i < n1; i += threads) out1[i] = in1[i] * f;
+  for (int64_t i = 4 * vecs + t; i < n; i += threads) out[i] = in[i] * f;
+}
+
+__global__ void __launch_bounds__(kScaleThreads)
+    k_scale_gradients(int64_t n0, const float* __restrict__ in0, float* __restrict__ out0,
+                      int64_t n1, const float* __restrict__ in1, float* __restrict__ out1,
+                      const float* __restrict__ factor) {
+  pdl_wait();
+  const float f = *factor;
+  scale_array(n0, in0, out0, f);
+  scale_array(n1, in1, out1, f);
 }
 
 int launch_scale_gradients(int64_t n0, const float* in0, float* out0, int64_t n1,
                            const float* in1, float* out1, const float* factor, cudaStream_t st) {
   if (n0 + n1 == 0) return GSB_OK;
-  const int64_t per = (int64_t)kScaleThreads * kScaleVec * 4;
-  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((n0 + per - 1) / per, 148 * 8));
+  const int64_t per = (int64_t)kScaleThreads * kScaleVec * 4, n = std::max(n0, n1);
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((n + per - 1) / per, 148 * 8));
   launch_pdl(k_scale_gradients, dim3((unsigned)blocks), dim3(kScaleThreads), 0, st, n0, in0, out0,
              n1, in1, out1, factor);
   return check_launch("scale_gradients");
