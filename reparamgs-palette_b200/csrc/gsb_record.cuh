@@ -9,11 +9,13 @@
 // With the conic scaled by -1/2 (exact), half_form gives p = -m / 2 of the
 // Mahalanobis form m bit for bit, the argument of exp(): alpha' = min(0.99,
 // alpha exp(min(p, 0))).  The reference skips a pixel whose alpha' is below
-// 0.002 (gsplatcu/kernel.cu:343-353).  expf is non-decreasing (checked for
-// every float in [-104, 0] on the device), and so is the rounded product with
-// alpha, so the pixels it skips are exactly those with p < p*, the smallest p
-// that is not skipped: one comparison decides, and the exponential is needed
-// only for its value.
+// 0.002 (gsplatcu/kernel.cu:343-353).  expf is non-decreasing over [-104, 0],
+// and so is the rounded product with alpha, so the pixels it skips are exactly
+// those with p < p*, the smallest p that is not skipped: one comparison
+// decides, and the exponential is needed only for its value.
+// tests/test_gpu_skip_threshold.py compares both float by float, around the
+// thresholds and over runs of consecutive floats, and allows no mismatch: run it
+// after a change of toolkit or of the math flags.
 //
 // Pixels outside the support box u +- (hx, hy) satisfy d^T Q d > c2, and any
 // pixel with d^T Q d > c2 is skipped: c2 = 2 ln(alpha/0.002) + margin, widened
