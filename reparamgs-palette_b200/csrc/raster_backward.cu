@@ -348,10 +348,11 @@ constexpr int kWild = 0x7fffffff;  // as a tile's largest contributor index
 // terms, for any channel count); dL/dT_final (vanilla_3dgs/gsplatcu/kernel.cu:
 // 912-919) enters as the value of R behind the last contributor, since
 // d T_final / d alpha' = -T_final / (1 - alpha').  As in the reference, the 0.99
-// clamp and max(0, .) are not differentiated.  Weights-only 8 blocks of 128
-// threads per SM (61 registers); full adjoint 7 for K = 4 and 5 (0.476 ->
-// 0.462 ms at 500k, K = 5, against 6), 6 otherwise (K = 3: 0.364 against 0.371
-// ms at 7; above 5 channels 7 would spill 90 bytes).
+// clamp and max(0, .) are not differentiated.  Weights-only at least 8 blocks of 128
+// threads per SM (61 registers above 5 channels; 56 up to 5, where 9 fit); full
+// adjoint 7 for K = 4 and 5 (500k: K = 4 0.513 against 0.519 ms at 6, K = 5 0.462
+// against 0.476), 6 otherwise (K = 3: 0.364 against 0.371 ms at 7; above 5 channels 7
+// would spill 90 bytes).
 template <int K, bool GEOM, int NP>
 __global__ void __launch_bounds__(AdjLayout<NP>::kThreads,
                                   (GEOM ? (K == 4 || K == 5 ? 7 : 6) : 8) * NP / 2)
@@ -565,11 +566,14 @@ __global__ void __launch_bounds__(kTilePixels)
   }
 }
 
-// Up to this many tiles (4 blocks per SM) a warp is alone on its scheduler or
-// nearly so, and the time is the longest tile's chain of records: with one
-// pixel per lane it is shorter (256 tiles, 20k Gaussians: 91 -> 63 us).  On
-// larger images the instructions count, 1.35x as many (1M Gaussians, 8160
-// tiles: 0.315 against 0.429 ms).
+// Up to this many tiles (4 blocks for each of 148 SMs) a warp is alone on its
+// scheduler or nearly so, and the time is the longest tile's chain of records: with
+// one pixel per lane it is shorter.  Two pixels / one, K = 5: 256 tiles, 20k Gaussians
+// 102 / 66 us (weights only 66 / 47), 80k 336 / 209; 432 tiles, 40k 168 / 109; 600
+// tiles, 60k 221 / 141, 240k 397 / 265.  On larger images the instructions count, 1.35x
+// as many, and the outcome depends on how long the longest list is: 1200 tiles, 600k
+// 385 / 308; 1900, 600k 367 / 371; 3600, 250k 285 / 261, 1M 455 / 531; 4346, 300k
+// 290 / 360; 8160, 1M weights only 315 / 429.  The line lies where one pixel always won.
 constexpr int kOnePixelTiles = 592;
 
 template <int K>

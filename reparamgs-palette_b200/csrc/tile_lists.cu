@@ -21,7 +21,8 @@
 // the serial part but multiply the counts (chunks x tiles words) that step 2 scans.
 // All steps together: 1M Gaussians, 3.3M patches, 1080p, 0.128 ms
 // (radix over patches: 0.169), of which the fill takes 0.054; 3M, 20.8M patches,
-// 4K, 0.56 ms (1.11), fill 0.36.
+// 4K, 0.56 ms (1.11), fill 0.36.  Every band reads its chunk's Gaussians, so an image
+// of many bands needs many patches per Gaussian to gain (the rule is in capi.cu).
 #include <algorithm>
 
 #include "gsb_common.cuh"
@@ -37,7 +38,7 @@ constexpr int kCountThreads = 512;
 constexpr int kCountCells = 48 * 1024;  // cells of a counting block (192 KB)
 constexpr int kRowGroup = 4;        // tile rows dealt to the bands at a time
 constexpr int kSplitWeight = 4;     // weight of a Gaussian besides its patches
-constexpr int kMaxChunks = 148;     // one block per SM and band
+constexpr int kMaxChunks = 148;     // one block per SM and band; sizes are asked for without a device
 
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
