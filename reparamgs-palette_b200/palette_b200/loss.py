@@ -28,21 +28,24 @@ import torch
 from gsplatcu import _lib
 
 
-def _dense(t, like):
-    """Is `t` a plain FP32 tensor whose elements lie in order in `like`'s device memory?
-    Not so: batched gradients (is_grads_batched, vectorised Jacobians: no storage),
-    tensor subclasses, and what a saved-tensor hook may hand back."""
-    return (type(t) is torch.Tensor and torch._C._has_storage(t) and t.is_cuda and
-            t.device == like.device and t.dtype == torch.float32 and t.is_contiguous())
+def _dense(t, device):
+    """Is `t` a plain FP32 tensor whose elements lie in order in the memory of CUDA
+    device number `device`?  Not so: tensor subclasses, and what a saved-tensor hook
+    may hand back."""
+    return (type(t) is torch.Tensor and t.dtype is torch.float32 and t.is_cuda and
+            t.get_device() == device and t.is_contiguous())
 
 
 def _times(g, first, second):
     """(first * g, second * g) for the incoming gradient `g`, a device scalar,
     in one launch; either may be None.  Under create_graph the products are
     torch's, so that they can be differentiated again, and so they are where
-    the library could not read a factor as it lies in memory."""
-    if first is None or torch.is_grad_enabled() or not all(
-            t is None or _dense(t, first) for t in (g, first, second)):
+    the library could not read a factor as it lies in memory: not dense FP32,
+    or a batched gradient (is_grads_batched, vectorised Jacobians: no storage)."""
+    if first is None or torch.is_grad_enabled() or not (
+            torch._C._has_storage(g) and _dense(g, first.get_device()) and
+            _dense(first, first.get_device()) and
+            (second is None or _dense(second, first.get_device()))):
         return (None if first is None else first * g, None if second is None else second * g)
     a = torch.empty_like(first)
     b = None if second is None else torch.empty_like(second)

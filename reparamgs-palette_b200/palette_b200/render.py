@@ -212,12 +212,14 @@ def _weight_args(shs, dc, A, B, K):
 def _check_rows(pws, rots, scales, alphas, w0, A, B, mode, K, P, Q, rank):
     """The kernels read (and the adjoint writes) pws.shape[0] rows of every
     parameter: refuse a tensor that holds fewer elements."""
-    n = int(pws.shape[0])
+    n = pws.shape[0]
+    full = mode == _lib.WEIGHTS_FULL
+    if (pws.numel() >= 3 * n and rots.numel() >= 4 * n and scales.numel() >= 3 * n and
+            alphas.numel() >= n and w0.numel() >= (16 * K if full else K) * n and
+            (full or (A.numel() >= P * rank * n and B.numel() >= rank * Q * n))):
+        return
     rows = [("pws", pws, 3), ("rots", rots, 4), ("scales", scales, 3), ("alphas", alphas, 1)]
-    if mode == _lib.WEIGHTS_FULL:
-        rows.append(("shs", w0, 16 * K))
-    else:
-        rows += [("dc", w0, K), ("A", A, P * rank), ("B", B, rank * Q)]
+    rows += [("shs", w0, 16 * K)] if full else [("dc", w0, K), ("A", A, P * rank), ("B", B, rank * Q)]
     for name, t, width in rows:
         if t.numel() < n * width:
             raise ValueError(f"render_palette: {name} {tuple(t.shape)} has fewer than {n} rows of "

@@ -36,7 +36,7 @@ from gsplatcu import _lib
 
 from .render import _check_rows, _params, _render_one, _weight_args, camera_struct
 
-_F32 = torch.float32
+_F32, _I32 = torch.float32, torch.int32
 
 # Low-rank shapes (K, P, Q, rank) of the fused kernels; full SH: K in 3..8.
 _FUSED_LOWRANK = {(5, 5, 15, 1), (5, 5, 15, 2), (5, 5, 15, 3), (5, 5, 15, 4), (3, 3, 15, 1),
@@ -58,9 +58,15 @@ def _operator_chain(pws, alphas, scales, rots, w0, A, B, cam, mode, K, Q):
     return layer, depths
 
 
+def _as_saved(t, dtype):
+    return t.dtype is dtype and t.is_cuda and t.is_contiguous()
+
+
 def _saved(t, dtype):
     """A tensor kept from the forward, as the library reads it: saved-tensor hooks
     may have handed back another layout (made dense) or type (refused)."""
+    if t is None:
+        return None
     if t.dtype != dtype or not t.is_cuda:
         raise TypeError(f"splat_palette_weights: a saved tensor came back as {t.dtype} on "
                         f"{t.device}, saved as {dtype} on a CUDA device")
@@ -92,12 +98,13 @@ class _SplatWeights(torch.autograd.Function):
                 f"splat_palette_weights: unsupported palette parameter shape (K={K}, P={P}, Q={Q}, "
                 f"rank={rank}) in the backward (status {_lib.GSB_ERR_UNSUPPORTED})",
                 _lib.GSB_ERR_UNSUPPORTED)
-        pws, tau = _saved(pws, _F32), _saved(tau, _F32)
-        state = _saved(state, torch.uint8)
-        if state.data_ptr() % 256:
-            state = state.clone()
-        ranges, gsid, contrib = (_saved(t, torch.int32) for t in (ranges, gsid, contrib))
-        w0, A, B = (None if t is None else _saved(t, wt) for t in (w0, A, B))
+        if not (_as_saved(pws, _F32) and _as_saved(tau, _F32) and _as_saved(state, torch.uint8) and
+                _as_saved(ranges, _I32) and _as_saved(gsid, _I32) and _as_saved(contrib, _I32) and
+                _as_saved(w0, wt) and (A is None or (_as_saved(A, wt) and _as_saved(B, wt))) and
+                state.data_ptr() % 256 == 0):
+            pws, tau, state = _saved(pws, _F32), _saved(tau, _F32), _saved(state, torch.uint8).clone()
+            ranges, gsid, contrib = _saved(ranges, _I32), _saved(gsid, _I32), _saved(contrib, _I32)
+            w0, A, B = _saved(w0, wt), _saved(A, wt), _saved(B, wt)
         dev = pws.device
         n = int(pws.shape[0])
         camst, _keep = camera_struct(cam)
