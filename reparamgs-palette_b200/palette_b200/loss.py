@@ -28,24 +28,21 @@ import torch
 from gsplatcu import _lib
 
 
-def _dense(t, device):
-    """Is `t` a plain FP32 tensor whose elements lie in order in the memory of CUDA
-    device number `device`?  Not so: tensor subclasses, and what a saved-tensor hook
-    may hand back."""
-    return (type(t) is torch.Tensor and t.dtype is torch.float32 and t.is_cuda and
-            t.get_device() == device and t.is_contiguous())
-
-
 def _times(g, first, second):
     """(first * g, second * g) for the incoming gradient `g`, a device scalar,
     in one launch; either may be None.  Under create_graph the products are
-    torch's, so that they can be differentiated again, and so they are where
-    the library could not read a factor as it lies in memory: not dense FP32,
-    or a batched gradient (is_grads_batched, vectorised Jacobians: no storage)."""
+    torch's, so that they can be differentiated again, and so they are where the
+    library could not read a factor as it lies in memory: a batched gradient
+    (is_grads_batched, vectorised Jacobians: no storage), a tensor subclass, and
+    what a saved-tensor hook may hand back in another layout, type or place."""
+    plain, f32 = torch.Tensor, torch.float32
     if first is None or torch.is_grad_enabled() or not (
-            torch._C._has_storage(g) and _dense(g, first.get_device()) and
-            _dense(first, first.get_device()) and
-            (second is None or _dense(second, first.get_device()))):
+            type(g) is plain and torch._C._has_storage(g) and g.dtype is f32 and
+            type(first) is plain and first.dtype is f32 and first.is_contiguous() and
+            first.is_cuda and g.get_device() == first.get_device() and
+            (second is None or (type(second) is plain and second.dtype is f32 and
+                                second.is_contiguous() and
+                                second.get_device() == first.get_device()))):
         return (None if first is None else first * g, None if second is None else second * g)
     a = torch.empty_like(first)
     b = None if second is None else torch.empty_like(second)
