@@ -31,7 +31,7 @@
 // passes, with three blocks per SM to fill them).  32x32 tiles that recomputed
 // their halo on every side and passed every sum through shared memory took
 // 0.220 ms at 1080p, K = 5, 0.113 at 720p and 0.024 at 256^2; this takes 0.134,
-// 0.069 and 0.022.  Two blocks per SM without spills 0.164; staging and gradients
+// 0.069 and 0.017 (the form for a block alone).  Two blocks per SM without spills 0.164; staging and gradients
 // on a third group of threads 0.176; a rolled row loop 0.16.
 #include <algorithm>
 #include <cmath>
@@ -174,13 +174,13 @@ __device__ __forceinline__ void ssim_h2(const ulonglong2* sMa, const float4* sMb
   sGb[rr * kPitchGb + run] = make_float4(b[0], b[1], b[2], b[3]);
 }
 
-// Stages step `b`: the image (from one read of the layer stack) and the target,
+// Stages a step: the image (from one read of the layer stack) and the target,
 // as (x, y) pairs, zero outside the image.  First image row `top`, column `left`.
-template <int K>
+template <int K, bool ALONE>
 __device__ __forceinline__ void ssim_stage(float2* sXY, const float* __restrict__ layer,
                                            const float* __restrict__ target, const float* sP,
                                            int H, int W, int64_t hw, int top, int left, int t) {
-#pragma unroll 1
+#pragma unroll (ALONE ? 3 : 1)
   for (int u = 0; u < (kSsimStep * kSsimXW + kSsimThreads - 1) / kSsimThreads; ++u) {
     const int e = t + u * kSsimThreads;
     if (e >= kSsimStep * kSsimXW) break;
@@ -209,9 +209,11 @@ __device__ __forceinline__ void ssim_sync() {
   asm volatile("barrier.sync %0, %1;" ::"n"(Id), "n"(Threads) : "memory");
 }
 
-// Grid: strips x segments of `rows` output rows each.
-template <int K, bool PAL>
-__global__ void __launch_bounds__(kSsimThreads, kSsimBlocks)
+// Grid: strips x segments of `rows` output rows each.  ALONE: a grid of at most one
+// block per SM, whose time is one block's chain of steps: it may use all registers and
+// has the loads of a step's staging and gradients in flight together.
+template <int K, bool PAL, bool ALONE>
+__global__ void __launch_bounds__(kSsimThreads, ALONE ? 1 : kSsimBlocks)
     k_palette_l1_ssim(int H, int W, int rows, const float* __restrict__ layer,
                       const float* __restrict__ palette, const float* __restrict__ target,
                       SsimWindow win, SsimScales sc, float* __restrict__ image,
@@ -255,7 +257,7 @@ __global__ void __launch_bounds__(kSsimThreads, kSsimBlocks)
 #pragma unroll 1
       for (int e = tid; e < kItemsH2; e += kSsimThreads) ssim_h2(sMa, sMb, sGa, sGb, g, e);
   };
-  ssim_stage<K>(reinterpret_cast<float2*>(sXY), layer, target, sP, H, W, hw, y0 - 2 * kSsimR,
+  ssim_stage<K, ALONE>(reinterpret_cast<float2*>(sXY), layer, target, sP, H, W, hw, y0 - 2 * kSsimR,
                 x0 - 2 * kSsimR, tid);
   auto sync = [] { ssim_sync<0, kSsimThreads>(); };
   const int lane = tid & 31, w = tid >> 5;
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(kSsimThreads, kSsimBlocks)
         }
       }
       if (s + 1 < steps)
-        ssim_stage<K>(reinterpret_cast<float2*>(sXY), layer, target, sP, H, W, hw,
+        ssim_stage<K, ALONE>(reinterpret_cast<float2*>(sXY), layer, target, sP, H, W, hw,
                       y0 - 2 * kSsimR + (s + 1) * kSsimStep, x0 - 2 * kSsimR, tid);
       sync();
     }
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(kSsimThreads, kSsimBlocks)
         }
         ssim_sync<1, kSsimRole>();
         const int top = y0 - 4 * kSsimR + (s - 1) * kSsimStep;  // output row of r = 0
-#pragma unroll 1
+#pragma unroll (ALONE ? 3 : 1)
         for (int u = 0; u < 3; ++u) {
           const int r = t / kSsimW + 4 * u, gy = top + r;
           if (r < kSsimStep && gx < W && gy >= y0 && gy < y1) {
@@ -395,7 +397,7 @@ __global__ void __launch_bounds__(kSsimThreads, kSsimBlocks)
         }
       }
       if (s + 1 < steps)
-        ssim_stage<K>(reinterpret_cast<float2*>(sXY), layer, target, sP, H, W, hw,
+        ssim_stage<K, ALONE>(reinterpret_cast<float2*>(sXY), layer, target, sP, H, W, hw,
                       y0 - 2 * kSsimR + (s + 1) * kSsimStep, x0 - 2 * kSsimR, tid);
       sync();
     }
@@ -441,7 +443,7 @@ __global__ void __launch_bounds__(kSsimThreads, kSsimBlocks)
   }
 }
 
-template <int K, bool PAL>
+template <int K, bool PAL, bool ALONE>
 static int launch_l1_ssim_k(dim3 grid, int rows, const float* layer, const float* palette,
                             const float* target, int H, int W, const SsimWindow& win,
                             const SsimScales& sc, float* image, float* loss, float* dlayer,
@@ -451,13 +453,13 @@ static int launch_l1_ssim_k(dim3 grid, int rows, const float* layer, const float
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !attr[dev]) {
-    if (cudaFuncSetAttribute(k_palette_l1_ssim<K, PAL>,
+    if (cudaFuncSetAttribute(k_palette_l1_ssim<K, PAL, ALONE>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kSsimSmemBytes) != cudaSuccess)
       return check_launch("palette_l1_ssim (shared memory attribute)", 0);
     if (dev >= 0 && dev < 64) attr[dev] = true;
   }
-  launch_pdl(k_palette_l1_ssim<K, PAL>, grid, dim3(kSsimThreads), kSsimSmemBytes, st, H, W,
+  launch_pdl(k_palette_l1_ssim<K, PAL, ALONE>, grid, dim3(kSsimThreads), kSsimSmemBytes, st, H, W,
              rows, layer, palette, target, win, sc, image, loss, dlayer, dpal);
   return check_launch("palette_l1_ssim");
 }
@@ -492,27 +494,44 @@ int launch_palette_l1_ssim(int K, int H, int W, const float* layer, const float*
   if (rc || hw == 0) return rc;
   // Segments of 11 s - 20 rows take s steps and one to finish; the blocks that
   // are resident at a time run in waves.  Take the s of the least waves x steps.
+  // Images whose segments of at most kAloneSteps steps fit on one block per SM take
+  // the fewest such steps instead, in the form for a block alone: three blocks that
+  // share an SM lengthen each other's steps, and at 80 registers they spill.  Shared /
+  // alone, K = 5 and 8: 100x100 15.2, 17.3 / 13.9, 14.0 us; 257x257 21.2, 24.8 / 17.2,
+  // 18.5; 300x300 21.4, 25.0 / 18.2, 20.3; 400x400 26.9, 32.0 / 25.0, 28.0; 2000x33
+  // 26.5, 30.4 / 21.2, 22.9 (32x32 tiles, one per SM here, took 21.3, 22.9).  With more
+  // steps the shared form wins: 640x480 32.9 / 35.8, 800x600 44.1 / 52.0.
+  constexpr int kAloneSteps = 6;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int64_t strips = (W + kSsimW - 1) / kSsimW, slots = (int64_t)sms * kSsimBlocks;
-  int rows = H;
-  int64_t best = -1;
-  for (int s = 4 * kSsimR / kSsimStep + 1;; ++s) {
+  const auto segments = [H](int s) {
     const int r = kSsimStep * s - 4 * kSsimR;
-    const int64_t segs = (H + r - 1) / r;
-    const int64_t cost = (strips * segs + slots - 1) / slots * (2 * s + 3);
-    if (segs <= 65535 && (best < 0 || cost < best)) best = cost, rows = r;
-    if (segs == 1) break;
+    return ((int64_t)H + r - 1) / r;
+  };
+  constexpr int kLeast = 4 * kSsimR / kSsimStep + 1;
+  int steps = kLeast;
+  while (steps < kAloneSteps && strips * segments(steps) > sms) ++steps;
+  const bool alone = strips * segments(steps) <= sms;
+  if (!alone) {
+    int64_t best = -1;
+    for (int s = kLeast;; ++s) {
+      const int64_t segs = segments(s), cost = (strips * segs + slots - 1) / slots * (2 * s + 3);
+      if (segs <= 65535 && (best < 0 || cost < best)) best = cost, steps = s;
+      if (segs == 1) break;
+    }
   }
+  const int rows = kSsimStep * steps - 4 * kSsimR;
   const dim3 grid((unsigned)strips, (unsigned)((H + rows - 1) / rows));
-  if (!palette) return launch_l1_ssim_k<3, false>(grid, rows, layer, nullptr, target, H, W, win, sc,
-                                                  image, loss, dlayer, nullptr, st);
+  if (!palette)
+    return (alone ? launch_l1_ssim_k<3, false, true> : launch_l1_ssim_k<3, false, false>)(
+        grid, rows, layer, nullptr, target, H, W, win, sc, image, loss, dlayer, nullptr, st);
   switch (K) {
 #define GSB_K(KK)                                                                          \
   case KK:                                                                                 \
-    return launch_l1_ssim_k<KK, true>(grid, rows, layer, palette, target, H, W, win, sc, image, \
-                                      loss, dlayer, dpal, st);
+    return (alone ? launch_l1_ssim_k<KK, true, true> : launch_l1_ssim_k<KK, true, false>)(  \
+        grid, rows, layer, palette, target, H, W, win, sc, image, loss, dlayer, dpal, st);
     GSB_K(1) GSB_K(2) GSB_K(3) GSB_K(4) GSB_K(5) GSB_K(6) GSB_K(7) GSB_K(8)
 #undef GSB_K
     default: return GSB_ERR_INVALID_ARGUMENT;
