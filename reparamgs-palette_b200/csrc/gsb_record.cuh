@@ -15,7 +15,10 @@
 // decides, and the exponential is needed only for its value.
 // tests/test_gpu_skip_threshold.py compares both float by float, around the
 // thresholds and over runs of consecutive floats, and allows no mismatch: run it
-// after a change of toolkit or of the math flags.
+// after a change of toolkit or of the math flags.  Outside of this are inputs that
+// no covariance and no sigmoid gives: conics above 1e37, whose m overflows at another
+// pixel than p, and an opacity of -infinity, which the reference blends as 0.99
+// where exp() underflows (-inf * 0 is NaN) and which never blends here.
 //
 // Pixels outside the support box u +- (hx, hy) satisfy d^T Q d > c2, and any
 // pixel with d^T Q d > c2 is skipped: c2 = 2 ln(alpha/0.002) + margin, widened
